@@ -315,12 +315,14 @@ int pv_rfi_bandpass_current(pv_rfi* rfi, float* h_out, int nbins, float* h_stats
  * band of nbins channels (256, 512 or 1024): partial p sums channels p,
  * p + parts, ... in order. */
 int pv_rfi_parts(int nbins);
-/* How pv_rfi_run spreads a band over the GPU (no counterpart in the
- * reference, whose clipper is one CPU thread): 0 one CTA of `parts`
- * threads; 1 (the default) bands of 1024 partials over a cluster of 4 CTAs
- * of 256 threads; 2 bands of 512 or 1024 partials over clusters of 128-thread
- * CTAs.  Every choice computes the same partial sums, so flags and outputs
- * are identical. */
+/* Makes pv_rfi_run walk the spectra one after another, and how that spreads a
+ * band over the GPU (no counterpart in the reference, whose clipper is one
+ * CPU thread): 0 one CTA of `parts` threads; 1 bands of 1024 partials over a
+ * cluster of 4 CTAs of 256 threads; 2 bands of 512 or 1024 partials over
+ * clusters of 128-thread CTAs.  Without this call a clipper whose RMS comes
+ * from the mean (compute_rms_from_mean) does its spectra in blocks, and one
+ * whose RMS does not walks them as with 1.  Every choice computes the same
+ * partial sums, so flags and outputs are identical. */
 int pv_rfi_set_split(pv_rfi* rfi, int split);
 
 /* ------------------------------------------------------------------------
@@ -441,10 +443,13 @@ typedef struct pv_batch pv_batch;
                                  the first chunk in which the channel varies (until then the
                                  channel's samples are stored as its offset) */
 /* How the clippers spread over the GPU.  Every choice computes the same
- * partial sums, so the flags and outputs are identical.  By default a
- * pipelined batch gives each beam's clipper one CTA (the clippers share the
- * GPU with the dedispersion) and an unpipelined batch spreads beams of more
- * than 4096 channels over a cluster of 4 CTAs (the clippers run alone). */
+ * partial sums, so the flags and outputs are identical.  By default a clipper
+ * whose RMS comes from the mean does its chunk's spectra in blocks, on the
+ * whole GPU.  Other clippers, and all of them with one of these flags, walk
+ * their spectra: without a flag, a pipelined batch gives each such beam one
+ * CTA (the clippers share the GPU with the dedispersion) and an unpipelined
+ * batch spreads beams of more than 4096 channels over a cluster of 4 CTAs
+ * (the clippers run alone). */
 #define PV_BATCH_RFI_ONE_CTA 64   /* one CTA per beam */
 #define PV_BATCH_RFI_CLUSTER8 128 /* beams of more than 1024 channels on clusters of 128-thread CTAs
                                      (4 CTAs up to 4096 channels, 8 beyond) */

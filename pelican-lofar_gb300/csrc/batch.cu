@@ -187,13 +187,17 @@ void destroy(pv_batch* b) {
     delete b;
 }
 
-// Issues one step of every beam on stream s.  Pipelined, the channeliser
-// runs first on the whole GPU.  Then the clippers (one CTA, one SM, per beam)
-// run on high-priority streams beside a persistent dedispersion launch with
-// one CTA for each SM they leave free; as each clipper class ends, a
-// dedispersion launch of as many CTAs joins the same tile queue on its
-// stream, so no SM idles and a dedispersion CTA never holds an SM a clipper
-// needs.  Both branches join s before the step counter advances.
+// Issues one step of every beam on stream s.  Clippers done in blocks of
+// spectra use the whole GPU for a few ms: their classes run side by side and
+// join s, and the ring write and the dedispersion follow on s.
+//
+// Beams whose spectra are walked hold one SM each for as long as a third of
+// the dedispersion.  Pipelined, those clippers run on high-priority streams
+// beside a persistent dedispersion launch with one CTA for each SM they leave
+// free; as each walked class ends, a dedispersion launch of as many CTAs
+// joins the same tile queue on its stream, so no SM idles and a dedispersion
+// CTA never holds an SM a clipper needs.  Both branches join s before the
+// step counter advances.
 int enqueue_step(pv_batch* b, cudaStream_t s, bool capture) {
     const bool timing = (b->flags & PV_BATCH_TIMING) != 0;
     auto mark = [&](int i, cudaStream_t st) -> int {
@@ -202,8 +206,11 @@ int enqueue_step(pv_batch* b, cudaStream_t s, bool capture) {
                                        : cudaEventRecord(b->ev[i], st),
                                "record stage event");
     };
-    cudaStream_t sd = b->pipelined ? b->side : s;      // dedispersion branch (low priority)
-    cudaStream_t sa = b->pipelined ? b->branch_a : s;  // clippers and ring write (high priority)
+    const int nc = b->rfi ? pv::rfi_batch_classes(b->rfi) : 0;
+    const int nb = b->rfi ? pv::rfi_batch_block_classes(b->rfi) : 0;  // classes 0..nb-1 in blocks, the rest walked
+    const bool beside = b->pipelined && nc > nb;  // walked clippers beside the dedispersion
+    cudaStream_t sd = beside ? b->side : s;      // dedispersion branch (low priority)
+    cudaStream_t sa = beside ? b->branch_a : s;  // walked clippers and ring write (high priority)
     plan_kernel<<<1, 256, 0, s>>>(b->d_bs, b->n, b->d_step, b->h_mask, b->pipelined ? 1 : 0);
     PV_TRY(pv::check_launch("plan_kernel"));
     PV_TRY(mark(0, s));
@@ -211,20 +218,30 @@ int enqueue_step(pv_batch* b, cudaStream_t s, bool capture) {
         PV_TRY(pv::launch_chan_fast(c.nchan, c.packets ? 2 : 1, c.d_jobs, pv::ChanJob{}, c.njobs, c.nwarps,
                                     b->d_bs, s));
     PV_TRY(mark(1, s));
-    const int nk = b->rfi ? pv::rfi_batch_launches(b->rfi) : 0;
+    // classes first..last-1 side by side, joined on s
+    auto classes = [&](int first, int last) -> int {
+        if (last - first > 1) PV_CUDA(cudaEventRecord(b->fork_ev, s), "fork");
+        for (int k = first + 1; k < last; ++k) {
+            PV_CUDA(cudaStreamWaitEvent(b->rfi_side[k - 1], b->fork_ev, 0), "fork clipper");
+            PV_TRY(pv::rfi_batch_launch_one(b->rfi, k, b->rfi_side[k - 1]));
+            PV_CUDA(cudaEventRecord(b->rfi_join[k - 1], b->rfi_side[k - 1]), "join clipper");
+        }
+        if (last > first) PV_TRY(pv::rfi_batch_launch_one(b->rfi, first, s));
+        for (int k = first + 1; k < last; ++k) PV_CUDA(cudaStreamWaitEvent(s, b->rfi_join[k - 1], 0), "join clipper");
+        return PV_OK;
+    };
+    PV_TRY(classes(0, nb));
     int rfi_ctas = 0;
-    for (int k = 0; k < nk; ++k) rfi_ctas += pv::rfi_batch_ctas(b->rfi, k);
-    if (b->pipelined) {
+    if (beside) {
+        for (int k = nb; k < nc; ++k) rfi_ctas += pv::rfi_batch_ctas(b->rfi, k);
         PV_TRY(pv::dd_batch_reset(b->dd, s));  // one tile queue for every dedispersion launch
         PV_CUDA(cudaEventRecord(b->fork_ev, s), "fork");
         PV_CUDA(cudaStreamWaitEvent(sa, b->fork_ev, 0), "fork");
         PV_CUDA(cudaStreamWaitEvent(sd, b->fork_ev, 0), "fork");
-    }
-    if (b->rfi && b->pipelined) {
-        // every clipper class resident at once (class 0 on branch A, the
+        // every walked class resident at once (the first on branch A, the
         // others on their own streams); as a class finishes, a dedispersion
         // launch of as many CTAs takes its SMs and joins the tile queue
-        for (int k = 1; k < nk; ++k) {
+        for (int k = nb + 1; k < nc; ++k) {
             cudaStream_t sk = b->rfi_side[k - 1];
             PV_CUDA(cudaStreamWaitEvent(sk, b->fork_ev, 0), "fork clipper");
             PV_TRY(pv::rfi_batch_launch_one(b->rfi, k, sk));
@@ -232,23 +249,15 @@ int enqueue_step(pv_batch* b, cudaStream_t s, bool capture) {
             PV_TRY(pv::dd_batch_launch_shared(b->dd, b->d_bs, pv::rfi_batch_ctas(b->rfi, k), sk));
             PV_CUDA(cudaEventRecord(b->rfi_tail[k - 1], sk), "join helper");
         }
-        if (nk > 0) PV_TRY(pv::rfi_batch_launch_one(b->rfi, 0, sa));
-        for (int k = 1; k < nk; ++k) PV_CUDA(cudaStreamWaitEvent(sa, b->rfi_join[k - 1], 0), "join clipper");
-    } else if (b->rfi) {
-        // the classes side by side, joined before the dedispersion
-        if (nk > 1) PV_CUDA(cudaEventRecord(b->fork_ev, s), "fork");
-        for (int k = 1; k < nk; ++k) {
-            PV_CUDA(cudaStreamWaitEvent(b->rfi_side[k - 1], b->fork_ev, 0), "fork clipper");
-            PV_TRY(pv::rfi_batch_launch_one(b->rfi, k, b->rfi_side[k - 1]));
-            PV_CUDA(cudaEventRecord(b->rfi_join[k - 1], b->rfi_side[k - 1]), "join clipper");
-        }
-        if (nk > 0) PV_TRY(pv::rfi_batch_launch_one(b->rfi, 0, s));
-        for (int k = 1; k < nk; ++k) PV_CUDA(cudaStreamWaitEvent(s, b->rfi_join[k - 1], 0), "join clipper");
+        PV_TRY(pv::rfi_batch_launch_one(b->rfi, nb, sa));
+        for (int k = nb + 1; k < nc; ++k) PV_CUDA(cudaStreamWaitEvent(sa, b->rfi_join[k - 1], 0), "join clipper");
+    } else {
+        PV_TRY(classes(nb, nc));
     }
     PV_TRY(mark(2, sa));
     auto dedisperse_branch = [&]() -> int {
         PV_TRY(mark(6, sd));
-        if (b->pipelined) {
+        if (beside) {
             // the SMs the clippers leave free; the clippers' SMs join later
             const int free_sms = std::max(8, pv::sm_count() - rfi_ctas);
             PV_TRY(pv::dd_batch_launch_shared(b->dd, b->d_bs, std::min(free_sms, pv::dd_batch_grid(b->dd)), sd));
@@ -269,18 +278,18 @@ int enqueue_step(pv_batch* b, cudaStream_t s, bool capture) {
         PV_TRY(pv::check_launch("event_export_kernel"));
         return mark(5, sd);
     };
-    if (b->pipelined) PV_TRY(dedisperse_branch());
+    if (beside) PV_TRY(dedisperse_branch());
     if (b->store == PV_STORE_U8)
         PV_TRY(pv::ring_calibrate_batch(b->d_ring_jobs, b->n, b->cal_blocks, b->d_bs, sa));
     PV_TRY(pv::ring_write_batch(b->d_ring_jobs, b->n, b->ring_blocks, b->d_bs, b->store, sa));
     PV_TRY(mark(3, sa));
-    if (b->pipelined) {
-        if (nk > 0) PV_TRY(pv::dd_batch_launch_shared(b->dd, b->d_bs, pv::rfi_batch_ctas(b->rfi, 0), sa));
+    if (beside) {
+        PV_TRY(pv::dd_batch_launch_shared(b->dd, b->d_bs, pv::rfi_batch_ctas(b->rfi, nb), sa));
         PV_CUDA(cudaEventRecord(b->join_a, sa), "join");
         PV_CUDA(cudaEventRecord(b->join_ev, sd), "join");
         PV_CUDA(cudaStreamWaitEvent(s, b->join_a, 0), "join");
         PV_CUDA(cudaStreamWaitEvent(s, b->join_ev, 0), "join");
-        for (int k = 1; k < nk; ++k) PV_CUDA(cudaStreamWaitEvent(s, b->rfi_tail[k - 1], 0), "join helper");
+        for (int k = nb + 1; k < nc; ++k) PV_CUDA(cudaStreamWaitEvent(s, b->rfi_tail[k - 1], 0), "join helper");
     } else {
         PV_TRY(dedisperse_branch());
     }
@@ -459,7 +468,9 @@ extern "C" int pv_batch_create(pv_batch** out, const pv_beam_config* configs, in
             nch[i] = b->beams[i]->nchan_fb;
         }
         rc = pv::rfi_batch_create(&b->rfi, hs.data(), data.data(), nsub.data(), nch.data(), nbeams,
-                                  chunk, b->d_bs, rfi_split(flags), s0);
+                                  chunk, b->d_bs, rfi_split(flags),
+                                  (flags & (PV_BATCH_RFI_ONE_CTA | PV_BATCH_RFI_CLUSTER8 | PV_BATCH_RFI_CLUSTER4)) != 0,
+                                  s0);
         if (rc != PV_OK) return fail(rc);
     }
     // A8: ring writes
@@ -547,7 +558,7 @@ extern "C" int pv_batch_create(pv_batch** out, const pv_beam_config* configs, in
             pv::set_error("pv_batch_create: cannot create streams");
             return fail(PV_ERR_CUDA);
         }
-        const int nk = b->rfi ? pv::rfi_batch_launches(b->rfi) : 0;
+        const int nk = b->rfi ? pv::rfi_batch_classes(b->rfi) : 0;
         for (int k = 1; k < nk; ++k) {
             b->rfi_side.push_back(nullptr);
             b->rfi_join.push_back(nullptr);
@@ -841,5 +852,6 @@ extern "C" long long pv_batch_footprint(const pv_beam_config* c, int flags) {
         bytes += 2LL * c->nsub * 2 * c->chunk * c->int_time * c->nchan_sub * 4;  // two input buffers
     bytes += 2LL * 2 * (long long)sizeof(float2) * c->nsub * 7 * c->nchan_sub;  // two PPF histories
     bytes += 16LL * c->history + 12LL * nbins;                        // clipper state, bandpass
+    bytes += pv::rfi_block_bytes(nbins);
     return bytes;
 }

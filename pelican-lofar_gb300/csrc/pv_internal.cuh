@@ -113,14 +113,17 @@ void dd_batch_destroy(DdBatch* b);
 // Batched RFI clippers (rfi.cu).
 struct RfiBatch;
 // handles[i] null: beam i has no clipper; bs: the batch's BeamStep array (inactive beams skip);
+// walk: every beam's spectra are walked (else only those of beams that cannot be done in blocks), spread by
 // split: 0 one CTA per beam; 1 beams of more than 4096 channels on a cluster of 4 CTAs;
 // 2 beams of more than 1024 channels on clusters of 128-thread CTAs
 int rfi_batch_create(RfiBatch** out, pv_rfi* const* handles, float* const* data, const int* nsub,
-                     const int* nchan, int n, int nt, const BeamStep* bs, int split, cudaStream_t s);
-int rfi_batch_launches(const RfiBatch* b);  // number of classes (beams with one channel count), largest first
+                     const int* nchan, int n, int nt, const BeamStep* bs, int split, bool walk, cudaStream_t s);
+int rfi_batch_classes(const RfiBatch* b);        // classes, those done in blocks first
+int rfi_batch_block_classes(const RfiBatch* b);  // how many of them are done in blocks
 int rfi_batch_launch_one(RfiBatch* b, int k, cudaStream_t s);
-int rfi_batch_ctas(const RfiBatch* b, int k);  // CTAs of class k (beams x CTAs per beam)
+int rfi_batch_ctas(const RfiBatch* b, int k);  // CTAs of walked class k (beams x CTAs per beam)
 void rfi_batch_destroy(RfiBatch* b);
+long long rfi_block_bytes(int nbins);  // device bytes of a clipper's block records
 
 // Batched ring writes (buffer.cu): stokes [nt][nsub][1][nchan] of one beam.
 struct RingJob {

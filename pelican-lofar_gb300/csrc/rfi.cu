@@ -3,8 +3,12 @@
 //
 // The clipper is a sequential state machine over spectra: every spectrum's
 // channel-clip margin, bandpass level and rejection test depend on running
-// averages updated by the previous spectrum.  One CTA, or for a wide beam a
-// cluster of CTAs, walks a beam's spectra in order; partial p (P = 256, 512
+// averages updated by the previous spectrum.  With the RMS taken from the mean
+// (computeRMSfromMean, the default) the spectra are done in blocks, all of a
+// block's spectra at once (rfi_blocks.cuh: 0.24 ms for 4096 spectra of 3904
+// channels).  Without it, or when a spread over CTAs is asked for, they are
+// walked (rfi_body: 24 ms): one CTA, or for a wide beam a cluster of CTAs,
+// takes a beam's spectra in order.  In both, partial p (P = 256, 512
 // or 1024 by channel count) owns channels p, p+P, ... of each spectrum.  The
 // state (running mean/RMS, their history rings, the last good spectrum, the
 // bandpass offset) lives in device memory between calls, so a stream of
@@ -15,7 +19,8 @@
 // bandpass are float as in the reference.  Channel sums use a fixed order
 // (partial p's sequential sum, a halving tree of offsets 16..1 inside each
 // warp, then offsets P/64..1 over the P/32 warp sums) so results are
-// deterministic and independent of how the partials are spread over CTAs.  Clip flags therefore match the reference's FP32 arithmetic
+// deterministic and independent of how the partials are spread over CTAs and
+// of the form.  Clip flags therefore match the reference's FP32 arithmetic
 // except for channels or spectra within rounding distance of a threshold.
 #include <algorithm>
 #include <cmath>
@@ -211,7 +216,9 @@ struct RfiState {
 struct RfiConfig {
     int nbins, history, zero_dming, use_mor, deg;
     float cr, sr, scale, mmm_f;
+    float term_abs;  // largest sum over channels of the k >= 1 terms' magnitudes
     double inv_sqrt_nbins;
+    double inv_h;  // 1 / history
 };
 
 struct RfiBuffers {
@@ -810,6 +817,8 @@ __device__ __forceinline__ void rfi_body(const RfiConfig& cfg, const RfiBuffers&
     if constexpr (C > 1) cooperative_groups::this_cluster().sync();  // no CTA leaves while others read it
 }
 
+#include "rfi_blocks.cuh"
+
 // T threads per CTA (which sets the register budget), C CTAs per beam (a
 // cluster); T * C is the partial count.
 template <int T, int C>
@@ -826,9 +835,98 @@ struct RfiJob {
     float* data;
     unsigned char* flags;
     Geo geo;
+    RfiWork work;
     int nt;
     int beam;  // index into the batch's BeamStep array
 };
+
+// Spectra [t0, t0 + n) of every job: jobs[blockIdx.y], or `one` when jobs is
+// null; beams without a chunk this step return at once.
+template <int P, int KM, bool PLAIN>
+__global__ void __launch_bounds__(P, P == 256 ? 6 : (P == 512 ? 3 : 1)) rfi_stats_kernel(const RfiJob* __restrict__ jobs,
+                                                      const __grid_constant__ RfiJob one,
+                                                      const pv::BeamStep* __restrict__ bs, int t0,
+                                                      bool second) {
+    const RfiJob& J = jobs ? jobs[blockIdx.y] : one;
+    if (bs && !bs[J.beam].active) return;
+    const long long spec_elems = (long long)J.geo.nsub * J.geo.npol * J.geo.nchan;
+    const int i = blockIdx.x;
+    rfi_stats_body<P, KM, PLAIN>(J.cfg, J.bufs, J.work, J.data + (long long)(t0 + i) * spec_elems, J.geo, i, second);
+}
+
+template <int P>
+__global__ void __launch_bounds__(kScanThreads, 1) rfi_scan_kernel(const RfiJob* __restrict__ jobs,
+                                                                   const __grid_constant__ RfiJob one,
+                                                                   const pv::BeamStep* __restrict__ bs, int t0,
+                                                                   int n, bool second) {
+    const RfiJob& J = jobs ? jobs[blockIdx.x] : one;
+    if (bs && !bs[J.beam].active) return;
+    const long long spec_elems = (long long)J.geo.nsub * J.geo.npol * J.geo.nchan;
+    rfi_scan_body<P>(J.cfg, J.bufs, J.work, J.data + (long long)t0 * spec_elems, J.geo, n, second);
+}
+
+// CTA 0 of a job adds up the fraction of bad channels, CTA 1 + i does spectrum i.
+template <int P, int KM, bool PLAIN>
+__global__ void __launch_bounds__(P, P == 256 ? 6 : (P == 512 ? 3 : 1)) rfi_apply_kernel(const RfiJob* __restrict__ jobs,
+                                                      const __grid_constant__ RfiJob one,
+                                                      const pv::BeamStep* __restrict__ bs, int t0, int n) {
+    const RfiJob& J = jobs ? jobs[blockIdx.y] : one;
+    if (bs && !bs[J.beam].active) return;
+    const int i = (int)blockIdx.x - 1;
+    if (i < 0) {
+        rfi_fraction<P>(J.cfg, J.bufs, J.work, n);
+        return;
+    }
+    const long long spec_elems = (long long)J.geo.nsub * J.geo.npol * J.geo.nchan;
+    rfi_apply_body<P, KM, PLAIN>(J.cfg, J.bufs, J.work, J.data + (long long)(t0 + i) * spec_elems, J.geo,
+                          J.flags ? J.flags + (long long)(t0 + i) * J.cfg.nbins : nullptr, i, i == n - 1);
+}
+
+template <int P, int KM, bool PLAIN>
+int rfi_blocks_t(const RfiJob* jobs, const RfiJob& one, int njobs, const pv::BeamStep* bs, int nt, cudaStream_t s) {
+    for (int t0 = 0; t0 < nt; t0 += kRfiBlock) {
+        const int n = std::min(kRfiBlock, nt - t0);
+        for (int second = 0; second < 2; ++second) {
+            rfi_stats_kernel<P, KM, PLAIN><<<dim3((unsigned)n, (unsigned)njobs), P, 0, s>>>(jobs, one, bs, t0, second);
+            PV_TRY(pv::check_launch("rfi_stats_kernel"));
+            rfi_scan_kernel<P><<<(unsigned)njobs, kScanThreads, 0, s>>>(jobs, one, bs, t0, n, second);
+            PV_TRY(pv::check_launch("rfi_scan_kernel"));
+        }
+        rfi_apply_kernel<P, KM, PLAIN><<<dim3((unsigned)n + 1, (unsigned)njobs), P, 0, s>>>(jobs, one, bs, t0, n);
+        PV_TRY(pv::check_launch("rfi_apply_kernel"));
+    }
+    return PV_OK;
+}
+
+// Channel counts that share the launches of rfi_blocks: the largest one of
+// the class (0x7fffffff: any number of channels per thread).
+int rfi_blocks_class(int nbins) {
+    for (int top : {1024, 4096, 8192, 16384})
+        if (nbins <= top) return top;
+    return 0x7fffffff;
+}
+// One polarisation and a flat bandpass: kernels without the general addressing
+// and bandpass, whose registers let a third more CTAs share an SM.
+bool rfi_plain(const RfiConfig& cfg, const RfiBuffers& bufs, int npol) {
+    return npol == 1 && cfg.deg == 0 && bufs.killed == nullptr;
+}
+
+// nt spectra of one beam (jobs null), or of the njobs beams of one class of a
+// batch; nbins is their largest channel count (or the class).
+template <bool PLAIN>
+int rfi_blocks_p(int nbins, const RfiJob* jobs, const RfiJob& one, int njobs, const pv::BeamStep* bs, int nt,
+                 cudaStream_t s) {
+    if (nbins <= 1024) return rfi_blocks_t<256, 4, PLAIN>(jobs, one, njobs, bs, nt, s);
+    if (nbins <= 4096) return rfi_blocks_t<512, 8, PLAIN>(jobs, one, njobs, bs, nt, s);
+    if (nbins <= 8192) return rfi_blocks_t<1024, 8, PLAIN>(jobs, one, njobs, bs, nt, s);
+    if (nbins <= 16384) return rfi_blocks_t<1024, 16, PLAIN>(jobs, one, njobs, bs, nt, s);
+    return rfi_blocks_t<1024, 0, PLAIN>(jobs, one, njobs, bs, nt, s);
+}
+int rfi_blocks(int nbins, bool plain, const RfiJob* jobs, const RfiJob& one, int njobs, const pv::BeamStep* bs, int nt,
+               cudaStream_t s) {
+    return plain ? rfi_blocks_p<true>(nbins, jobs, one, njobs, bs, nt, s)
+                 : rfi_blocks_p<false>(nbins, jobs, one, njobs, bs, nt, s);
+}
 
 // The clippers of many beams at once: cluster b (CTAs b*C .. b*C+C-1) runs
 // job b (every job of a launch has the same partial count); beams without a
@@ -942,7 +1040,9 @@ struct pv_rfi {
     Bandpass bp;
     float cr = 10.0f, sr = 4.0f;
     int history = 10, zero_dming = 0, use_mor = 1, band_matching = 0, active = 1;
-    int split = 1;  // rfi_shape's split of a wide beam over a cluster
+    int split = 1;  // rfi_shape's split of a wide beam over a cluster (the walk over spectra)
+    bool walk = false;  // pv_rfi_set_split was called: the walk, spread as asked
+    RfiWork work{};
     float start_freq = 0.0f, end_freq = 0.0f;
     int nbins = 0;
     RfiConfig cfg{};
@@ -963,10 +1063,17 @@ void free_device(pv_rfi* h) {
     if (h->dev.last_good) cudaFree(h->dev.last_good);
     if (h->d_terms) cudaFree(h->d_terms);
     if (h->d_killed) cudaFree(h->d_killed);
+    if (h->work.rec) cudaFree(h->work.rec);  // one allocation
+    h->work = RfiWork{};
     h->dev = RfiBuffers{};
     h->d_terms = nullptr;
     h->d_killed = nullptr;
 }
+
+// The block launches need the RMS history to follow from the mean: with
+// computeRMSfromMean off it takes each spectrum's RMS after flattening, whose
+// last bits follow the bandpass of that spectrum, and the spectra are walked.
+bool rfi_in_blocks(const pv_rfi* h) { return h->use_mor != 0 && !h->walk; }
 
 // First run with this channel count: rebin the model (RFI_Clipper.cpp:184-187)
 // and set up the device state.
@@ -989,10 +1096,16 @@ int setup(pv_rfi* h, int nbins, cudaStream_t s) {
     std::vector<float> terms((size_t)std::max(deg, 0) * nbins);
     std::vector<unsigned char> killed(nbins, 0);
     bool any_killed = false;
+    float term_abs = 0.0f;
     const float scale = (float)(h->bp.current.width / h->bp.primary.width);
     for (int i = 0; i < nbins; ++i) {
         const float v = (float)m.value(i);
-        for (int k = 1; k <= deg; ++k) terms[(size_t)(k - 1) * nbins + i] = h->bp.params[k] * powi(v, k);
+        float sum = 0.0f;
+        for (int k = 1; k <= deg; ++k) {
+            terms[(size_t)(k - 1) * nbins + i] = h->bp.params[k] * powi(v, k);
+            sum += std::fabs(terms[(size_t)(k - 1) * nbins + i]);
+        }
+        if (!(sum <= term_abs)) term_abs = sum;
     }
     // channels the kill list zeroes stay zero in every rebuilt model
     {
@@ -1014,6 +1127,8 @@ int setup(pv_rfi* h, int nbins, cudaStream_t s) {
     h->cfg.scale = scale;
     h->cfg.mmm_f = (float)(4.0f / std::sqrt(2.0 * 4.0f));  // k/sqrt(2k), k = 4 degrees of freedom
     h->cfg.inv_sqrt_nbins = 1.0 / std::sqrt((double)nbins);
+    h->cfg.term_abs = term_abs;
+    h->cfg.inv_h = 1.0 / (double)h->history;
     RfiState st{};
     st.remaining_zeros = nbins;
     st.params0 = h->bp.params[0];
@@ -1023,6 +1138,15 @@ int setup(pv_rfi* h, int nbins, cudaStream_t s) {
     PV_CUDA(cudaMalloc(&h->dev.mean_buf, sizeof(double) * h->history), "allocate RFI history");
     PV_CUDA(cudaMalloc(&h->dev.rms_buf, sizeof(double) * h->history), "allocate RFI history");
     PV_CUDA(cudaMalloc(&h->dev.last_good, sizeof(float) * nbins), "allocate RFI last good spectrum");
+    if (rfi_in_blocks(h)) {
+        const size_t head = (sizeof(SpecRec) + sizeof(SpecOut)) * kRfiBlock;
+        char* p = nullptr;
+        PV_CUDA(cudaMalloc(&p, head + sizeof(int) * ((size_t)nbins + kHdrWords)), "allocate RFI block records");
+        h->work.rec = reinterpret_cast<SpecRec*>(p);
+        h->work.out = reinterpret_cast<SpecOut*>(p + sizeof(SpecRec) * kRfiBlock);
+        h->work.hdr = reinterpret_cast<int*>(p + head);
+        h->work.fill_at = h->work.hdr + kHdrWords;
+    }
     PV_CUDA(cudaMemcpyAsync(h->dev.state, &st, sizeof(st), cudaMemcpyHostToDevice, s), "copy RFI state");
     PV_CUDA(cudaMemsetAsync(h->dev.last_good, 0, sizeof(float) * nbins, s), "clear last good spectrum");
     PV_CUDA(cudaMemsetAsync(h->dev.mean_buf, 0, sizeof(double) * h->history, s), "clear history");
@@ -1109,6 +1233,10 @@ extern "C" int pv_rfi_run(pv_rfi* h, float* d_data, int nt, int nsub, int npol, 
         return PV_ERR_ARG;
     }
     const Geo geo = make_geo(nsub, npol, nchan);
+    if (rfi_in_blocks(h) && h->work.rec) {
+        const RfiJob one{h->cfg, h->dev, d_data, d_flags, geo, h->work, nt, 0};
+        return rfi_blocks(nbins, rfi_plain(h->cfg, h->dev, npol), nullptr, one, 1, nullptr, nt, s);
+    }
     return rfi_launch(parts, h->split, smem, 1, nullptr, nullptr, h->cfg, h->dev, d_data, nt, geo, d_flags, s);
 }
 
@@ -1161,6 +1289,7 @@ extern "C" int pv_rfi_set_split(pv_rfi* h, int split) {
         return PV_ERR_ARG;
     }
     h->split = split;
+    h->walk = true;
     return PV_OK;
 }
 
@@ -1226,13 +1355,19 @@ extern "C" int pv_rfi_bandpass(pv_rfi* h, float* out, int nbins) {
 }
 
 // ---------------------------------------------------------------------------
-// Batched clippers: the RFI_Clipper of every beam of a batch, one CTA per
-// beam, one launch per class of beams with the same channel count (so the
-// same partial-sum count and about the same time per spectrum): the SMs of a
-// class are free for other work as soon as its own beams are done.  Classes
-// run largest channel count first.
+// Batched clippers: the RFI_Clipper of every beam of a batch.  Beams done in
+// blocks of spectra (rfi_in_blocks) form one class per partial count and
+// register budget.  Beams whose spectra are walked form one class per channel
+// count (so the same partial-sum count and about the same time per spectrum):
+// the SMs of a class are free for other work as soon as its own beams are
+// done.  Classes run largest channel count first, those in blocks before the
+// walked ones.
 // ---------------------------------------------------------------------------
 namespace pv {
+
+long long rfi_block_bytes(int nbins) {
+    return (long long)(sizeof(SpecRec) + sizeof(SpecOut)) * kRfiBlock + 4LL * (nbins + kHdrWords);
+}
 
 struct RfiBatch {
     struct Class {
@@ -1240,8 +1375,11 @@ struct RfiBatch {
         size_t smem = 0;
         RfiJob* d_jobs = nullptr;
         int njobs = 0;
+        bool blocks = false, plain = false;
     };
     std::vector<Class> classes;
+    int nblocks = 0;  // classes done in blocks, the first ones
+    int nt = 0;
     const BeamStep* bs = nullptr;
     int split = 1;
 };
@@ -1254,15 +1392,19 @@ void rfi_batch_destroy(RfiBatch* b) {
 }
 
 int rfi_batch_create(RfiBatch** out, pv_rfi* const* handles, float* const* data, const int* nsub,
-                     const int* nchan, int n, int nt, const BeamStep* bs, int split, cudaStream_t s) {
+                     const int* nchan, int n, int nt, const BeamStep* bs, int split, bool walk,
+                     cudaStream_t s) {
     auto* b = new RfiBatch;
     b->bs = bs;
+    b->nt = nt;
     b->split = split;
     std::vector<std::vector<RfiJob>> jobs;
     for (int i = 0; i < n; ++i) {
         pv_rfi* h = handles[i];
         if (!h || !h->active) continue;
         const int nbins = nsub[i] * nchan[i];
+        if (walk) h->walk = true;
+        const bool blocks = rfi_in_blocks(h);
         int rc = setup(h, nbins, s);
         const int parts = pv_rfi_parts(nbins);
         int T = 0, C = 0;
@@ -1277,11 +1419,18 @@ int rfi_batch_create(RfiBatch** out, pv_rfi* const* handles, float* const* data,
             return rc;
         }
         size_t k = 0;
-        while (k < b->classes.size() && b->classes[k].nbins != nbins) ++k;
+        const int key = blocks ? rfi_blocks_class(nbins) : nbins;
+        const bool plain = blocks && rfi_plain(h->cfg, h->dev, 1);
+        while (k < b->classes.size() &&
+               (b->classes[k].blocks != blocks || b->classes[k].plain != plain || b->classes[k].nbins != key))
+            ++k;
         if (k == b->classes.size()) {
             b->classes.emplace_back();
             b->classes[k].parts = parts;
-            b->classes[k].nbins = nbins;
+            b->classes[k].nbins = key;
+            b->classes[k].blocks = blocks;
+            b->classes[k].plain = plain;
+            if (blocks) ++b->nblocks;
             b->classes[k].threads = T;
             b->classes[k].ctas = C;
             jobs.emplace_back();
@@ -1293,15 +1442,19 @@ int rfi_batch_create(RfiBatch** out, pv_rfi* const* handles, float* const* data,
         j.data = data[i];
         j.flags = nullptr;
         j.geo = make_geo(nsub[i], 1, nchan[i]);
+        j.work = h->work;
         j.nt = nt;
         j.beam = i;
         jobs[k].push_back(j);
     }
-    {  // largest channel count first
+    {  // in blocks first, then largest channel count first
         std::vector<size_t> order(b->classes.size());
         for (size_t k = 0; k < order.size(); ++k) order[k] = k;
         std::stable_sort(order.begin(), order.end(),
-                         [&](size_t x, size_t y) { return b->classes[x].nbins > b->classes[y].nbins; });
+                         [&](size_t x, size_t y) {
+                             const RfiBatch::Class &p = b->classes[x], &q = b->classes[y];
+                             return p.blocks != q.blocks ? p.blocks : p.nbins > q.nbins;
+                         });
         std::vector<RfiBatch::Class> cs;
         std::vector<std::vector<RfiJob>> js;
         for (size_t k : order) {
@@ -1320,7 +1473,7 @@ int rfi_batch_create(RfiBatch** out, pv_rfi* const* handles, float* const* data,
                            cudaMemcpyHostToDevice);
         int rc = e == cudaSuccess ? PV_OK : cuda_status(e, "RFI batch jobs");
         // set the kernel attribute now, outside any stream capture
-        if (rc == PV_OK)
+        if (rc == PV_OK && !c.blocks)
             rc = rfi_launch(c.parts, b->split, c.smem, 0, c.d_jobs, nullptr, RfiConfig{}, RfiBuffers{}, nullptr, 0,
                             Geo{}, nullptr, s);
         if (rc != PV_OK) {
@@ -1332,13 +1485,16 @@ int rfi_batch_create(RfiBatch** out, pv_rfi* const* handles, float* const* data,
     return PV_OK;
 }
 
-int rfi_batch_launches(const RfiBatch* b) { return (int)b->classes.size(); }
+int rfi_batch_classes(const RfiBatch* b) { return (int)b->classes.size(); }
+
+int rfi_batch_block_classes(const RfiBatch* b) { return b->nblocks; }
 
 int rfi_batch_ctas(const RfiBatch* b, int k) { return b->classes[k].njobs * b->classes[k].ctas; }
 
 int rfi_batch_launch_one(RfiBatch* b, int k, cudaStream_t s) {
     auto& c = b->classes[k];
     if (c.njobs == 0) return PV_OK;
+    if (c.blocks) return rfi_blocks(c.nbins, c.plain, c.d_jobs, RfiJob{}, c.njobs, b->bs, b->nt, s);
     return rfi_launch(c.parts, b->split, c.smem, c.njobs, c.d_jobs, b->bs, RfiConfig{}, RfiBuffers{}, nullptr, 0,
                       Geo{}, nullptr, s);
 }

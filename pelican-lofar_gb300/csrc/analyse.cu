@@ -6,11 +6,18 @@
 // records every value at or above level n's threshold.  Events are listed
 // after a dummy (0,0,1,0) by DM, block, level and position.
 //
-// One thread owns one (DM, block) pair: it loads the 2^P samples, builds the
-// tree in registers with the reference's pairing (bit-identical sums) and
-// counts its events.  An exclusive scan over the pairs in (DM, block) order
-// gives every pair its output offset, and a second pass rebuilds the tree and
-// writes the events in the reference order.
+// Two launches.  The (DM, block) pairs in the reference's order are cut into
+// tiles of 128.  analyse_count reads every sample once, a warp 128 adjacent
+// samples at a time (16 bytes per lane), builds the tree in the lanes with the
+// reference's pairing (bit-identical sums) and leaves each tile's number of
+// events; the CTA that finishes last turns these into the tiles' places in the
+// list.  analyse_emit does the few tiles that have events over again, a thread
+// per pair, and writes them in order.
+//
+// Bound: HBM, one read of the window (134 MB for 2048 x 16384: 20 us at the
+// measured copy rate).  Before, a thread read its own block's 256 bytes, four
+// more launches scanned one count per pair, and the 6 MB of counts were
+// allocated and given back on every pv_analyse call: 390 us for that call.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -74,149 +81,237 @@ __device__ __forceinline__ void walk_block(float (&b)[1 << P], const Thresholds&
     TreeLevel<P, 1, F>::run(b, thr, emit);
 }
 
-template <int P>
-__global__ void analyse_count(const float* __restrict__ data, long long ld, int tdms, int nblocks,
-                              Thresholds thr, bool vec4, int* __restrict__ counts) {
-    const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long npairs = (long long)tdms * nblocks;
-    if (g >= npairs) return;
-    const int dm = (int)(g / nblocks), i = (int)(g % nblocks);
-    float b[1 << P];
-    load_block<P>(b, data + dm * ld + (long long)i * (1 << P), vec4);
-    int n = 0;
-    walk_block<P>(b, thr, [&](int, int, float) { ++n; });
-    counts[g] = n;
-}
+constexpr int kTilePairs = 128;      // (DM, block) pairs of a tile
+constexpr int kCountThreads = 256;
 
-template <int P>
-__global__ void analyse_emit(const float* __restrict__ data, long long ld, int tdms, int nblocks,
-                             Thresholds thr, bool vec4, const int* __restrict__ counts,
-                             const long long* __restrict__ offsets, pv_event* __restrict__ ev,
-                             long long cap) {
-    const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (g == 0 && cap > 0) ev[0] = pv_event{0, 0, 1.0f, 0.0f};
-    const long long npairs = (long long)tdms * nblocks;
-    if (g >= npairs || counts[g] == 0) return;
-    const int dm = (int)(g / nblocks), i = (int)(g % nblocks);
-    float b[1 << P];
-    load_block<P>(b, data + dm * ld + (long long)i * (1 << P), vec4);
-    long long o = 1 + offsets[g];
-    const int base = i * (1 << P);
-    walk_block<P>(b, thr, [&](int t, int w, float v) {
-        if (o < cap) ev[o] = pv_event{dm, base + t, (float)w, v};
-        ++o;
-    });
-}
+// Device scratch of one call, laid out by tiles_in().
+struct Tiles {
+    long long* offset;  // [tiles] events before the tile's first
+    int* count;         // [tiles]
+    unsigned* done;     // CTAs finished; 0 between calls
+};
 
-// ---------------------------------------------------------------------------
-// Exclusive scan of n values into long long offsets (1024 per block, block
-// totals scanned recursively).
-// ---------------------------------------------------------------------------
-constexpr int kScanBlock = 1024;
-
-template <typename T>
-__global__ void scan_block(const T* __restrict__ in, long long* __restrict__ out,
-                           long long* __restrict__ block_sums, long long n) {
-    __shared__ long long warp_tot[32];
-    const long long g = blockIdx.x * (long long)kScanBlock + threadIdx.x;
-    const long long v = g < n ? (long long)in[g] : 0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    long long x = v;
+// Runs in every CTA after it has stored its count: the last one to get here
+// scans the counts of all tiles and leaves the total (with the dummy event).
+__device__ __forceinline__ void finish_tiles(const Tiles& w, int ntiles, long long* total) {
+    __shared__ bool last;
+    __shared__ long long wsum[kCountThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        __threadfence();
+        last = atomicAdd(w.done, 1u) == (unsigned)gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!last) return;
+    const int per = (ntiles + kCountThreads - 1) / kCountThreads;
+    const int first = min(tid * per, ntiles), end = min(first + per, ntiles);
+    long long sum = 0;
+    for (int i = first; i < end; ++i) sum += __ldcg(w.count + i);
+    long long x = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const long long y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
-    if (lane == 31) warp_tot[warp] = x;
+    if (lane == 31) wsum[warp] = x;
     __syncthreads();
-    if (warp == 0) {
-        long long w = warp_tot[lane];
+    long long at = x - sum;
+    for (int k = 0; k < warp; ++k) at += wsum[k];
+    for (int i = first; i < end; ++i) {
+        w.offset[i] = at;
+        at += __ldcg(w.count + i);
+    }
+    if (tid == kCountThreads - 1) *total = 1 + at;
+    if (tid == 0) *w.done = 0;
+}
+
+// Rows of 16-byte aligned samples, blocks of 8 to 256.  Lane l holds samples
+// 4l..4l+3 of a group of 128; a block of 2^P samples is 2^(P-2) lanes, and the
+// levels above 2 add lane pairs (the upper lane of a pair gets the same sum,
+// which is not counted).  For P == 8 a block is two groups.
+template <int P>
+__global__ void __launch_bounds__(kCountThreads) analyse_count_vec(const float* __restrict__ data, long long ld,
+                                                                   int nblocks, long long npairs, Thresholds thr,
+                                                                   Tiles w, int ntiles, long long* total) {
+    constexpr int M = 1 << P, G = P == 8 ? 2 : 1;    // 128-sample groups that a warp takes together
+    constexpr int LANES = P == 8 ? 32 : M / 4;       // lanes of a block within a group
+    constexpr int NW = kCountThreads / 32;
+    constexpr int GROUPS = kTilePairs * M / (128 * G);  // of a tile
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long long g0 = (long long)blockIdx.x * kTilePairs;
+    const int dm0 = (int)(g0 / nblocks), i0 = (int)(g0 - (long long)dm0 * nblocks);
+    const int left = (int)min((long long)kTilePairs, npairs - g0);
+    int n = 0;
+    constexpr int UNROLL = GROUPS / NW >= 4 ? 4 : (GROUPS / NW >= 2 ? 2 : 1);
+#pragma unroll 1
+    for (int q0 = warp; q0 < GROUPS; q0 += NW * UNROLL) {
+        float4 v[UNROLL][G];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const long long y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
+        for (int u = 0; u < UNROLL; ++u) {
+            const int q = q0 + u * NW;
+            const int p = P == 8 ? q : (q * 128 + 4 * lane) / M;  // the lane's pair within the tile
+            int i = i0 + p, dm = dm0;
+            if (i >= nblocks) {
+                const int r = i / nblocks;
+                dm += r;
+                i -= r * nblocks;
+            }
+            const float4* src = reinterpret_cast<const float4*>(data + (long long)dm * ld + (long long)i * M);
+#pragma unroll
+            for (int h = 0; h < G; ++h)
+                v[u][h] = p < left ? __ldcs(src + h * 32 + (P == 8 ? lane : lane % LANES))
+                                   : make_float4(NAN, NAN, NAN, NAN);  // never at a threshold
         }
-        warp_tot[lane] = w;  // inclusive over warps
+#pragma unroll
+        for (int u = 0; u < UNROLL; ++u) {
+            float top[G];
+#pragma unroll
+            for (int h = 0; h < G; ++h) {
+                const float4 x = v[u][h];
+                n += (x.x >= thr.v[0]) + (x.y >= thr.v[0]) + (x.z >= thr.v[0]) + (x.w >= thr.v[0]);
+                const float a = __fadd_rn(x.x, x.y), b = __fadd_rn(x.z, x.w);
+                n += (a >= thr.v[1]) + (b >= thr.v[1]);
+                float c = __fadd_rn(a, b);
+                n += c >= thr.v[2];
+#pragma unroll
+                for (int k = 3; k <= (P == 8 ? 7 : P); ++k) {
+                    const int bit = 1 << (k - 3);
+                    const float o = __shfl_xor_sync(0xffffffffu, c, bit);
+                    c = __fadd_rn(c, o);  // commutative: both lanes hold the lower + upper sum
+                    n += (lane & (2 * bit - 1)) == 0 && c >= thr.v[k];
+                }
+                top[h] = c;
+            }
+            if (P == 8) n += lane == 0 && __fadd_rn(top[0], top[G - 1]) >= thr.v[8];
+        }
     }
+    n = __reduce_add_sync(0xffffffffu, n);
+    __shared__ int part[NW];
+    if (lane == 0) part[warp] = n;
     __syncthreads();
-    const long long before = warp == 0 ? 0 : warp_tot[warp - 1];
-    if (g < n) out[g] = before + x - v;
-    if (threadIdx.x == kScanBlock - 1) block_sums[blockIdx.x] = warp_tot[31];
-}
-
-__global__ void scan_add(long long* __restrict__ out, const long long* __restrict__ block_off,
-                         long long n) {
-    const long long g = blockIdx.x * (long long)kScanBlock + threadIdx.x;
-    if (g < n && blockIdx.x > 0) out[g] += block_off[blockIdx.x];
-}
-
-// total = 1 (the dummy) + events of every (DM, block) pair
-__global__ void analyse_total(const int* __restrict__ counts, const long long* __restrict__ offsets,
-                              long long npairs, long long* __restrict__ total) {
-    *total = npairs > 0 ? 1 + offsets[npairs - 1] + counts[npairs - 1] : 1;
-}
-
-// Block sums and their scans of every level of the scan of n values.
-constexpr long long scan_workspace(long long n) {
-    return n > 1 ? 2 * ((n + kScanBlock - 1) / kScanBlock) + scan_workspace((n + kScanBlock - 1) / kScanBlock)
-                 : 0;
-}
-
-// Scratch bytes of the analyser for npairs (trial, block) pairs: per-pair
-// counts and offsets, the scan workspace and two totals, rounded to 256.
-constexpr size_t scratch_bytes_for(long long npairs) {
-    return (((size_t)(npairs > 1 ? npairs : 1) * (sizeof(int) + sizeof(long long)) +
-             (size_t)(scan_workspace(npairs > 1 ? npairs : 1) + 2) * sizeof(long long) + 256) + 255) /
-           256 * 256;
-}
-
-// Exclusive scan of in[0..n) into out; ws holds scan_workspace(n) values.
-template <typename T>
-int exclusive_scan(const T* in, long long* out, long long n, long long* ws, cudaStream_t s) {
-    const long long nb = pv::ceil_div<long long>(n, kScanBlock);
-    long long* sums = ws;
-    long long* sums_scan = ws + nb;
-    scan_block<T><<<(unsigned)nb, kScanBlock, 0, s>>>(in, out, sums, n);
-    PV_TRY(pv::check_launch("scan_block"));
-    if (nb > 1) {
-        PV_TRY(exclusive_scan<long long>(sums, sums_scan, nb, ws + 2 * nb, s));
-        scan_add<<<(unsigned)nb, kScanBlock, 0, s>>>(out, sums_scan, n);
-        PV_TRY(pv::check_launch("scan_add"));
+    if (tid == 0) {
+        int t = 0;
+        for (int k = 0; k < NW; ++k) t += part[k];
+        w.count[blockIdx.x] = t;
     }
-    return PV_OK;
+    finish_tiles(w, ntiles, total);
+}
+
+// Any alignment and block size: a thread per pair.
+template <int P>
+__global__ void __launch_bounds__(kCountThreads) analyse_count(const float* __restrict__ data, long long ld,
+                                                               int nblocks, long long npairs, Thresholds thr,
+                                                               Tiles w, int ntiles, long long* total) {
+    const int tid = threadIdx.x;
+    const long long g = (long long)blockIdx.x * kTilePairs + tid;
+    int n = 0;
+    if (tid < kTilePairs && g < npairs) {
+        const int dm = (int)(g / nblocks), i = (int)(g % nblocks);
+        float b[1 << P];
+        load_block<P>(b, data + dm * ld + (long long)i * (1 << P), false);
+        walk_block<P>(b, thr, [&](int, int, float) { ++n; });
+    }
+    __shared__ int sum;
+    if (tid == 0) sum = 0;
+    __syncthreads();
+    n = __reduce_add_sync(0xffffffffu, n);
+    if ((tid & 31) == 0 && n) atomicAdd(&sum, n);
+    __syncthreads();
+    if (tid == 0) w.count[blockIdx.x] = sum;
+    finish_tiles(w, ntiles, total);
+}
+
+// CTA t writes tile t's events; CTA 0 the dummy event as well.
+template <int P>
+__global__ void __launch_bounds__(kTilePairs) analyse_emit(const float* __restrict__ data, long long ld, int nblocks,
+                                                           long long npairs, Thresholds thr, bool vec4, Tiles w,
+                                                           pv_event* __restrict__ ev, long long cap) {
+    __shared__ int wsum[kTilePairs / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (blockIdx.x == 0 && tid == 0 && cap > 0) ev[0] = pv_event{0, 0, 1.0f, 0.0f};
+    if (npairs == 0 || w.count[blockIdx.x] == 0) return;
+    const long long g = (long long)blockIdx.x * kTilePairs + tid;
+    const int dm = (int)(g / nblocks), i = (int)(g % nblocks);
+    const float* src = data + dm * ld + (long long)i * (1 << P);
+    float b[1 << P];
+    int n = 0;
+    if (g < npairs) {
+        load_block<P>(b, src, vec4);
+        walk_block<P>(b, thr, [&](int, int, float) { ++n; });
+    }
+    int x = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    if (n == 0) return;
+    long long o = 1 + w.offset[blockIdx.x] + x - n;
+    for (int k = 0; k < warp; ++k) o += wsum[k];
+    const int base = i * (1 << P);
+    load_block<P>(b, src, vec4);
+    walk_block<P>(b, thr, [&](int t, int width, float v) {
+        if (o < cap) ev[o] = pv_event{dm, base + t, (float)width, v};
+        ++o;
+    });
+}
+
+__global__ void analyse_none(pv_event* ev, long long cap, long long* total) {
+    if (cap > 0) ev[0] = pv_event{0, 0, 1.0f, 0.0f};
+    *total = 1;
+}
+
+// Scratch bytes of the analyser for npairs (trial, block) pairs, rounded to
+// 256: what is placed after it stays aligned.
+constexpr long long tiles_of(long long npairs) {
+    return npairs > 0 ? (npairs + kTilePairs - 1) / kTilePairs : 1;
+}
+constexpr size_t scratch_bytes_for(long long npairs) {
+    return ((size_t)tiles_of(npairs) * (sizeof(int) + sizeof(long long)) + 16 + 255) / 256 * 256;
+}
+// The counter comes first, at the same place for every size.
+Tiles tiles_in(void* p, long long npairs) {
+    Tiles w;
+    w.done = static_cast<unsigned*>(p);
+    w.offset = reinterpret_cast<long long*>(static_cast<char*>(p) + 16);
+    w.count = reinterpret_cast<int*>(w.offset + tiles_of(npairs));
+    return w;
 }
 
 template <int P>
-int run_analyse(const float* data, long long ld, int tdms, int nsamp, const Thresholds& thr,
-                pv_event* ev, long long cap, long long* d_total, int* counts, long long* offsets,
-                long long* ws, cudaStream_t s) {
+int run_analyse(const float* data, long long ld, int tdms, int nsamp, const Thresholds& thr, pv_event* ev,
+                long long cap, long long* d_total, void* scratch, cudaStream_t s) {
     const int nblocks = nsamp >> P;
     const long long npairs = (long long)tdms * nblocks;
-    const bool vec4 = (ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(data) & 15) == 0);
-    const int threads = 128;
-    if (npairs > 0) {
-        const unsigned blocks = (unsigned)pv::ceil_div<long long>(npairs, threads);
-        analyse_count<P><<<blocks, threads, 0, s>>>(data, ld, tdms, nblocks, thr, vec4, counts);
-        PV_TRY(pv::check_launch("analyse_count"));
-        PV_TRY(exclusive_scan<int>(counts, offsets, npairs, ws, s));
-        analyse_emit<P><<<blocks, threads, 0, s>>>(data, ld, tdms, nblocks, thr, vec4, counts,
-                                                   offsets, ev, cap);
-        PV_TRY(pv::check_launch("analyse_emit"));
-    } else if (cap > 0) {
-        analyse_emit<P><<<1, 32, 0, s>>>(data, ld, tdms, 0, thr, false, counts, offsets, ev, cap);
-        PV_TRY(pv::check_launch("analyse_emit"));
+    if (npairs == 0) {
+        analyse_none<<<1, 1, 0, s>>>(ev, cap, d_total);
+        return pv::check_launch("analyse_none");
     }
-    analyse_total<<<1, 1, 0, s>>>(counts, offsets, npairs, d_total);
-    return pv::check_launch("analyse_total");
+    const Tiles w = tiles_in(scratch, npairs);
+    const bool vec4 = (ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(data) & 15) == 0);
+    const int ntiles = (int)tiles_of(npairs);
+    // blocks of fewer than 8 samples are too short for the lanes' tree to have a level
+    if constexpr (P >= 3) {
+        if (vec4)
+            analyse_count_vec<P><<<ntiles, kCountThreads, 0, s>>>(data, ld, nblocks, npairs, thr, w, ntiles, d_total);
+    }
+    if (P < 3 || !vec4)
+        analyse_count<P><<<ntiles, kCountThreads, 0, s>>>(data, ld, nblocks, npairs, thr, w, ntiles, d_total);
+    PV_TRY(pv::check_launch("analyse_count"));
+    analyse_emit<P><<<ntiles, kTilePairs, 0, s>>>(data, ld, nblocks, npairs, thr, vec4, w, ev, cap);
+    return pv::check_launch("analyse_emit");
 }
 
 }  // namespace
 
 namespace pv {
 
-// Scratch bytes the analyser needs for tdms x nsamp at 2^bin_pow2 blocks.
+// Scratch bytes the analyser needs for tdms x nsamp at 2^bin_pow2 blocks.  It
+// has to be cleared once; every call leaves its counter at 0.
 size_t analyse_scratch_bytes(int tdms, int nsamp, int bin_pow2) {
-    // rounded to 256 bytes: keeps anything placed after it aligned
     return scratch_bytes_for((long long)tdms * (nsamp >> bin_pow2));
 }
 
@@ -227,16 +322,9 @@ int analyse_launch(const float* data, long long ld, int tdms, int nsamp, float t
                    void* scratch, cudaStream_t s) {
     Thresholds thr{};
     PV_TRY(pv_analyser_thresholds(threshold, rms, bin_pow2, thr.v));
-    const long long npairs = std::max<long long>((long long)tdms * (nsamp >> bin_pow2), 1);
-    char* p = static_cast<char*>(scratch);
-    long long* offsets = reinterpret_cast<long long*>(p);
-    p += npairs * sizeof(long long);
-    long long* ws = reinterpret_cast<long long*>(p);
-    p += (scan_workspace(npairs) + 2) * sizeof(long long);
-    int* counts = reinterpret_cast<int*>(p);
     switch (bin_pow2) {
 #define PV_CASE(P) \
-    case P: return run_analyse<P>(data, ld, tdms, nsamp, thr, ev, cap, d_total, counts, offsets, ws, s);
+    case P: return run_analyse<P>(data, ld, tdms, nsamp, thr, ev, cap, d_total, scratch, s);
         PV_CASE(0) PV_CASE(1) PV_CASE(2) PV_CASE(3) PV_CASE(4) PV_CASE(5) PV_CASE(6) PV_CASE(7)
         PV_CASE(8)
 #undef PV_CASE
@@ -275,19 +363,19 @@ extern "C" int pv_analyse(const float* d_data, long long ld, int tdms, int nsamp
         return PV_ERR_ARG;
     }
     cudaStream_t s = pv::as_stream(stream);
-    void* scratch = nullptr;
-    PV_TRY(pv::scratch_alloc(&scratch, pv::analyse_scratch_bytes(tdms, nsamp, bin_pow2) + 64, s));
-    long long* d_total = reinterpret_cast<long long*>(static_cast<char*>(scratch) +
-                                                      pv::analyse_scratch_bytes(tdms, nsamp, bin_pow2));
-    int rc = pv::analyse_launch(d_data, ld, tdms, nsamp, threshold, rms, bin_pow2, d_events, cap,
-                                d_total, scratch, s);
-    if (rc == PV_OK) {
-        rc = pv::cuda_status(cudaMemcpyAsync(h_count, d_total, sizeof(long long),
-                                             cudaMemcpyDeviceToHost, s), "read event count");
-        if (rc == PV_OK) rc = pv::cuda_status(cudaStreamSynchronize(s), "synchronise");
+    pv::Scratch scratch;
+    PV_TRY(pv::scratch_take(&scratch, pv::analyse_scratch_bytes(tdms, nsamp, bin_pow2)));
+    // the total goes straight to host memory
+    int rc = pv::analyse_launch(d_data, ld, tdms, nsamp, threshold, rms, bin_pow2, d_events, cap, scratch.host,
+                                scratch.dev, s);
+    if (rc == PV_OK) rc = pv::cuda_status(cudaStreamSynchronize(s), "synchronise");
+    if (rc != PV_OK) {  // its kernels may not have run to their end
+        pv::scratch_drop(scratch);
+        return rc;
     }
-    pv::scratch_free(scratch, s);
-    return rc;
+    *h_count = *static_cast<volatile long long*>(scratch.host);
+    pv::scratch_give(scratch);
+    return PV_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -301,7 +389,7 @@ constexpr size_t kNoAllocPairs = PV_ANALYSE_NOALLOC_MAX_PAIRS;
 constexpr size_t kNoAllocScratch = scratch_bytes_for((long long)kNoAllocPairs);
 static_assert(scratch_bytes_for((long long)kNoAllocPairs) >= scratch_bytes_for((long long)kNoAllocPairs - 1),
               "scratch grows with the pair count");
-// Scratch (counts, offsets, scan workspace) followed by the event total.
+// Scratch (counts, offsets, counter) followed by the event total.
 // Every GPU that loads the library keeps this array until the process exits.
 __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratch + 256];
 
@@ -356,8 +444,8 @@ extern "C" int pv_analyse_noalloc(const float* d_data, long long ld, int tdms, i
     }
     void* scratch = nullptr;
     PV_TRY(noalloc_scratch(&scratch));
-    // Nothing in the scratch needs clearing: the launch writes every count,
-    // offset, workspace entry and the total before it reads them.
+    // Nothing in the scratch needs clearing: every count, offset and the total are written before they
+    // are read, and the counter is 0 between calls.
     long long* d_total = reinterpret_cast<long long*>(static_cast<char*>(scratch) + kNoAllocScratch);
     cudaStream_t s = pv::as_stream(stream);
     PV_TRY(pv::analyse_launch(d_data, ld, tdms, nsamp, threshold, rms, bin_pow2, d_events, cap,

@@ -90,6 +90,8 @@ int beam_create(pv_beam** out, const pv_beam_config* c, int extra, int elem) {
     alloc((void**)&b->d_out, sizeof(float) * (size_t)c->tdms * c->chunk);
     alloc((void**)&b->d_events, sizeof(pv_event) * (size_t)b->cap);
     alloc(&b->d_scratch, scratch + 256);
+    if (e == cudaSuccess) e = cudaMemset(b->d_scratch, 0, scratch + 256);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);  // the beam's stream may not wait for it
     if (e == cudaSuccess) e = cudaMallocHost((void**)&b->h_total, sizeof(long long));
     if (e == cudaSuccess)
         e = cudaMemset(b->d_ring, elem == 1 ? 0x80 : 0, (size_t)elem * b->nbins * (size_t)b->row_stride);

@@ -75,9 +75,17 @@ cudaError_t allow_max_dynamic_smem(Kernel kern, size_t* limit = nullptr) {
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
 }
 
-// Stream-ordered scratch allocation (cudaMallocAsync / cudaFreeAsync).
-int scratch_alloc(void** p, size_t bytes, cudaStream_t s);
-void scratch_free(void* p, cudaStream_t s);
+// Scratch of a call that waits for its work before it returns: device memory
+// (cleared when it was allocated) and 64 bytes of host memory that kernels can
+// write.  scratch_give wants it idle; scratch_drop frees it.
+struct Scratch {
+    void* dev = nullptr;
+    long long* host = nullptr;
+    size_t bytes = 0;
+};
+int scratch_take(Scratch* out, size_t bytes);
+void scratch_give(const Scratch& b);
+void scratch_drop(const Scratch& b);
 
 }  // namespace pv
 

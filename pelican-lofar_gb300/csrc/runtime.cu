@@ -13,6 +13,19 @@ namespace {
 thread_local char t_error[512] = "";
 std::mutex g_sm_mutex;
 std::vector<int> g_sm_counts;
+
+// Blocks of scratch that calls have given back, per device: at most
+// kScratchKeep of them and kScratchBytes in all.  A call that waits for its
+// result gives its block back idle, so the next one takes it as it is;
+// cudaMallocAsync and cudaFreeAsync around the same call cost 0.2 ms where
+// another copy on the stream followed (the analyser's event list).
+constexpr size_t kScratchKeep = 8, kScratchBytes = 16u << 20;
+std::mutex g_scratch_mutex;
+struct Kept {
+    int device;
+    Scratch block;
+};
+std::vector<Kept> g_scratch;
 }  // namespace
 
 std::atomic<long long> g_launches{0};
@@ -50,19 +63,54 @@ int smem_optin() {
     return n;
 }
 
-int scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
-    *p = nullptr;
-    if (bytes == 0) return PV_OK;
-    cudaError_t e = cudaMallocAsync(p, bytes, s);
+int scratch_take(Scratch* out, size_t bytes) {
+    int dev = 0;
+    PV_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
+    {
+        std::lock_guard<std::mutex> lk(g_scratch_mutex);
+        for (size_t i = 0; i < g_scratch.size(); ++i)
+            if (g_scratch[i].device == dev && g_scratch[i].block.bytes >= bytes) {
+                *out = g_scratch[i].block;
+                g_scratch.erase(g_scratch.begin() + (long)i);
+                return PV_OK;
+            }
+    }
+    Scratch b;
+    b.bytes = bytes < 65536 ? 65536 : bytes;
+    cudaError_t e = cudaMalloc(&b.dev, b.bytes);
+    if (e == cudaSuccess) e = cudaMemset(b.dev, 0, b.bytes);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);  // the caller's stream may not wait for it
+    if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&b.host), 64, cudaHostAllocMapped);
     if (e != cudaSuccess) {
         set_error("scratch allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+        scratch_drop(b);
         return PV_ERR_NOMEM;
     }
+    *out = b;
     return PV_OK;
 }
 
-void scratch_free(void* p, cudaStream_t s) {
-    if (p) cudaFreeAsync(p, s);
+void scratch_give(const Scratch& b) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) {
+        std::lock_guard<std::mutex> lk(g_scratch_mutex);
+        size_t n = 0, total = b.bytes;
+        for (const Kept& k : g_scratch)
+            if (k.device == dev) {
+                ++n;
+                total += k.block.bytes;
+            }
+        if (n < kScratchKeep && total <= kScratchBytes) {
+            g_scratch.push_back({dev, b});
+            return;
+        }
+    }
+    scratch_drop(b);
+}
+
+void scratch_drop(const Scratch& b) {
+    if (b.dev) cudaFree(b.dev);
+    if (b.host) cudaFreeHost(b.host);
 }
 
 }  // namespace pv

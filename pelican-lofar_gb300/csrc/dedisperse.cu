@@ -19,6 +19,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <map>
+#include <mutex>
 #include <vector>
 
 #include <cuda_fp16.h>
@@ -67,6 +68,21 @@ struct DedispArgs {
     int stall;                   // failure-path test: the first stage's copies are withheld
 };
 
+// Linear rows: the first position of the buffer that channel c's row does not
+// read.  Contiguous rows (row_len == row_stride, the DedispersionBuffer layout)
+// read on into the next row as the reference kernel does; only reads past the
+// whole buffer become zeros.
+__device__ __forceinline__ long long linear_end(const DedispArgs& a, int c) {
+    return a.row_len == a.row_stride ? (long long)a.nchan * a.row_stride : (long long)c * a.row_stride + a.row_len;
+}
+
+// x mod n for x >= 0; mostly below 2n.
+__device__ __forceinline__ long long ring_column(long long x, long long n) {
+    if (x < n) return x;
+    x -= n;
+    return x < n ? x : x % n;
+}
+
 template <int DMS, int R, int CS>
 __global__ void __launch_bounds__(DMS * 32)
 dedisperse_kernel(const DedispArgs a) {
@@ -103,13 +119,8 @@ dedisperse_kernel(const DedispArgs a) {
                     cp_async4(dst + j, src + g);
                 }
             } else {
-                // Contiguous rows (row_len == row_stride, the DedispersionBuffer
-                // layout) read on into the next row as the reference kernel
-                // does; only reads past the whole buffer become zeros.
                 const long long g0 = t0 + s0;
-                const long long lim = a.row_len == a.row_stride
-                                          ? (long long)(a.nchan - c) * a.row_stride
-                                          : a.row_len;
+                const long long lim = linear_end(a, c) - (long long)c * a.row_stride;
                 for (int j = threadIdx.x; j < span; j += NT) {
                     const long long g = g0 + j;
                     if (g < lim) cp_async4(dst + j, src + g);
@@ -225,7 +236,7 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
 
 
 template <int DMS, int R, int CS, int ST>
-__global__ void __launch_bounds__((DMS + 1) * 32, 1)
+__global__ void __launch_bounds__((DMS + 1) * 32)
 dedisperse_tma_kernel(const DedispArgs a, int* __restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int TT = 32 * R;
@@ -263,7 +274,14 @@ dedisperse_tma_kernel(const DedispArgs a, int* __restrict__ status) {
         const int valid = (int)min((long long)TT, (long long)a.nout - t0);
         int issued = 0;
         bool ok = true;
+        const bool mine = lane < CS;
+        // the next stage's delay constants are on their way while this stage waits for its slot
+        float k_next = mine && lane < a.nchan ? a.dmshift[lane] : 0.0f;
+        const long long col0 = a.ring_len > 0 ? (a.t_base + t0) % a.ring_len : t0;
         for (int st = 0; st < nstages && ok; ++st) {
+            const float k = k_next;
+            const int cn = (st + 1) * CS + lane;
+            if (mine && cn < a.nchan) k_next = a.dmshift[cn];
             const int b = st % ST;
             const unsigned round = (unsigned)(st / ST);
             if (!mbar_wait_warp(&empty[b], (round & 1u) ^ 1u, a.wait_ns)) {
@@ -278,19 +296,42 @@ dedisperse_tma_kernel(const DedispArgs a, int* __restrict__ status) {
             const int c = st * CS + lane;
             unsigned bytes = 0, piece1 = 0, piece2 = 0;
             long long g_al = 0;
-            if (lane < CS && c < a.nchan) {
-                const float k = a.dmshift[c];
+            int tail = 0;  // linear rows: samples from piece1 on that are not copied in bulk
+            if (mine && c < a.nchan) {
                 const int s0 = pv_shift(k, dv0);
                 const int span = valid + pv_shift(k, dv_last) - s0;
-                const long long g0 = (a.t_base + t0 + s0) % a.ring_len;
-                g_al = g0 & ~3LL;
-                const int base = (int)(g0 - g_al);
-                const unsigned n = (unsigned)((base + span + 3) & ~3);
-                piece1 = (unsigned)min((long long)n, a.ring_len - g_al);
-                piece2 = n - piece1;
-                bytes = n * 4u;
+                int base;
+                if (a.ring_len > 0) {
+                    const long long g0 = ring_column(col0 + s0, a.ring_len);
+                    g_al = g0 & ~3LL;
+                    base = (int)(g0 - g_al);
+                    const unsigned n = (unsigned)((base + span + 3) & ~3);
+                    piece1 = (unsigned)min((long long)n, a.ring_len - g_al);
+                    piece2 = n - piece1;
+                } else {
+                    // Positions in the whole buffer: aligned units up to the last readable sample
+                    // (linear_end), the rest one by one, zeros beyond it.
+                    const long long g0 = (long long)c * a.row_stride + t0 + s0;
+                    g_al = g0 & ~3LL;
+                    base = (int)(g0 - g_al);
+                    const long long end = linear_end(a, c), want = (base + span + 3) & ~3;
+                    const long long fit = end > g_al ? (end - g_al) & ~3LL : 0;
+                    piece1 = (unsigned)min(want, fit);
+                    tail = max(0, base + span - (int)piece1);
+                }
+                bytes = (piece1 + piece2) * 4u;
                 meta_off[b * CS + lane] = s0 - base;
                 meta_k[b * CS + lane] = k;
+                __threadfence_block();
+            }
+            for (unsigned m = __ballot_sync(0xffffffffu, tail > 0); m; m &= m - 1) {
+                const int l = __ffs(m) - 1;
+                const int first = __shfl_sync(0xffffffffu, (int)piece1, l), n = __shfl_sync(0xffffffffu, tail, l);
+                const long long g = __shfl_sync(0xffffffffu, g_al, l) + first;
+                const long long end = linear_end(a, st * CS + l);
+                float* dst = slots + (size_t)(b * CS + l) * a.slot + first;
+                for (int j = lane; j < n; j += 32) dst[j] = g + j < end ? a.in[g + j] : 0.0f;
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                 __threadfence_block();
             }
             unsigned total = bytes;
@@ -300,9 +341,9 @@ dedisperse_tma_kernel(const DedispArgs a, int* __restrict__ status) {
             if (lane == 0) mbar_arrive_expect_tx(&full[b], total);
             __syncwarp();
             if (bytes) {
-                const float* src = a.in + (long long)c * a.row_stride;
+                const float* src = a.ring_len > 0 ? a.in + (long long)c * a.row_stride : a.in;
                 float* dst = slots + (size_t)(b * CS + lane) * a.slot;
-                bulk_g2s(dst, src + g_al, piece1 * 4u, &full[b]);
+                if (piece1) bulk_g2s(dst, src + g_al, piece1 * 4u, &full[b]);
                 if (piece2) bulk_g2s(dst + piece1, src, piece2 * 4u, &full[b]);
             }
             issued = st + 1;
@@ -460,11 +501,19 @@ __device__ __forceinline__ void batch_producer(const pv::DdJob* __restrict__ job
         const float dv0 = pv_trial_value(tt.d0, J.start, J.step);
         const float dv_last = pv_trial_value(d_last, J.start, J.step);
         const int valid = min(TT, J.nout - tt.t0);
-        const long long t_base = (bs[J.beam].window * J.chunk) % J.ring_len;
+        const long long col0 = (bs[J.beam].window * J.chunk + tt.t0) % J.ring_len;
         const int nst = (J.nchan + CS - 1) / CS;
+        const bool mine = lane < CS;
+        const float* dmshift = J.dmshift;
+        const int nchan = J.nchan;
+        const long long ring_len = J.ring_len;
+        float k_next = mine && lane < nchan ? dmshift[lane] : 0.0f;
         const unsigned char* ring = reinterpret_cast<const unsigned char*>(J.ring);
         for (int st = 0; st < nst; ++st) {
             const int b = gs % ST;
+            const float k = k_next;  // the next stage's are on their way while this one waits for its slot
+            const int cn = (st + 1) * CS + lane;
+            if (mine && cn < nchan) k_next = dmshift[cn];
             if (st > 0 && !mbar_wait_warp(&empty[b], ((gs / ST) & 1u) ^ 1u, wait_ns)) {
                 if (lane == 0) atomicExch(status, PV_ERR_TIMEOUT);
                 ok = false;
@@ -474,15 +523,14 @@ __device__ __forceinline__ void batch_producer(const pv::DdJob* __restrict__ job
             const int c = st * CS + lane;
             unsigned bytes = 0, piece1 = 0, piece2 = 0;
             long long g_al = 0;
-            if (lane < CS && c < J.nchan) {
-                const float k = J.dmshift[c];
+            if (mine && c < nchan) {
                 const int s0 = pv_shift(k, dv0);
                 const int span = valid + pv_shift(k, dv_last) - s0;
-                const long long g0 = (t_base + tt.t0 + s0) % J.ring_len;
+                const long long g0 = ring_column(col0 + s0, ring_len);
                 g_al = g0 & ~(long long)(AU - 1);
                 const int base = (int)(g0 - g_al);
                 const unsigned n = (unsigned)((base + span + AU - 1) & ~(AU - 1));
-                piece1 = (unsigned)min((long long)n, J.ring_len - g_al);
+                piece1 = (unsigned)min((long long)n, ring_len - g_al);
                 piece2 = n - piece1;
                 bytes = n * (unsigned)E;
                 meta_off[b * CS + lane] = s0 - base;
@@ -998,41 +1046,87 @@ static size_t tma_smem(int st, int cs, int slot_floats) {
     return (size_t)st * cs * slot_floats * sizeof(float) + (size_t)st * cs * 8 + 8 + 2 * st * 8;
 }
 
+// Tiles of the pipelined kernel: trials x samples, channels per stage, stages.
+struct TmaTile {
+    int dms, tt, cs, st;
+    float rate;  // adds per second with every SM busy, of the first one's
+};
+// Tadd/s on 512 trials x 3904 channels x 16384 samples (110-158 MHz, DM 125:
+// tile spreads of 16 trials up to 1050 samples) / 512 x 512 x 10976 / 300 x
+// 496 x 5003 / 512 x 512 x 1024 (up to 120), fetching the delay constants one
+// stage ahead:
+//   16 x 1024, 8 x 2   7.84  6.76  4.94  1.70
+//    8 x 1024, 8 x 2   6.57  7.85  4.86  2.33
+//    8 x  256, 16 x 2  4.37  7.43  6.21  4.02
+// Wide tiles need the fewest copied samples per add, narrow ones fill the SMs
+// where the wide ones are few; 16 x 4 in 2-channel stages holds spreads that
+// 8-channel stages do not.
+constexpr TmaTile kTmaTiles[] = {{16, 1024, 8, 2, 1.0f}, {16, 1024, 2, 4, 0.93f}, {8, 1024, 8, 2, 0.95f},
+                                 {8, 256, 16, 2, 0.93f}};
+
+// The tile with the least expected time, -1 if none fits: the busiest SM's
+// share of the adds, at a rate that falls where a tile copies more than 0.55
+// bytes per add through L2.
+template <typename F>
+int tma_tile(int tdms, int nout, long long ring_len, F spread) {
+    int best = -1;
+    double best_t = 0.0;
+    for (int v = 0; v < 4; ++v) {
+        const TmaTile& t = kTmaTiles[v];
+        const int sp = spread(t.dms);
+        if (tma_smem(t.st, t.cs, (t.tt + sp + 8 + 3) & ~3) > 220 * 1024) continue;
+        // every copy (span + 16-byte rounding) must fit in one ring turn
+        if (ring_len > 0 && ring_len < (long long)std::min(t.tt, nout) + sp + 8) continue;
+        const double tiles = (double)ceil_div(tdms, t.dms) * ceil_div(nout, t.tt);
+        const double busiest = std::ceil(tiles / sm_count());
+        const double copied = 4.0 * (t.tt + sp) / ((double)t.tt * t.dms);
+        const double time = busiest * t.dms * t.tt / t.rate * std::max(1.0, copied / 0.55);
+        if (best < 0 || time < best_t) {
+            best = v;
+            best_t = time;
+        }
+    }
+    return best;
+}
+
 // Chooses the tile for the delay spread: the widest trial tile whose channel
-// slots fit in shared memory with two buffers of CS channels.
+// slots fit in shared memory with two buffers of CS channels.  spread(dms) is
+// the largest delay spread of dms trials (delay_spread).
+template <typename F>
 int dedisperse_device(float* out, long long out_stride, const float* in, long long row_stride,
                       long long row_len, long long ring_len, long long t_base, int nchan, int nout,
-                      int tdms, const float* d_dmshift, const std::vector<float>& h_dmshift,
-                      float start, float step, cudaStream_t s, int* status) {
+                      int tdms, const float* d_dmshift, F spread, float start, float step, cudaStream_t s,
+                      int* status) {
     if (ring_len > 0 && (ring_len > row_stride || t_base < 0)) {
         set_error("dedispersion: ring of %lld samples does not fit rows of %lld", ring_len, row_stride);
         return PV_ERR_ARG;
     }
     DedispArgs a{out, out_stride, in, row_stride, row_len, ring_len, t_base % std::max(ring_len, 1LL),
                  d_dmshift, nchan, nout, tdms, start, step, 0, wait_ns(), 0};
-    // Ring rows with 16-byte aligned spans go through the TMA pipeline.
-    if (status && ring_len > 0 && ring_len % 4 == 0 && row_stride % 4 == 0 &&
-        (reinterpret_cast<uintptr_t>(in) & 15) == 0 && getenv("PV_DEDISP_V1") == nullptr) {
-        a.stall = take_stall();
-        const int spread16 = delay_spread(h_dmshift, tdms, 16, start, step);
-        const int slot = (1024 + spread16 + 8 + 3) & ~3;
-        // every copy (span + 16-byte rounding) must fit in one ring turn
-        const bool fits = ring_len >= (long long)std::min(1024, nout) + spread16 + 8;
-        if (fits && tma_smem(4, 4, slot) <= 220 * 1024)
-            return launch_dedisperse_tma<16, 32, 4, 4>(a, spread16, status, s);
-        if (fits && tma_smem(4, 2, slot) <= 220 * 1024)
-            return launch_dedisperse_tma<16, 32, 2, 4>(a, spread16, status, s);
+    // Rows whose 16-byte units bulk copies can fetch go through the pipeline.
+    const bool aligned = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
+    const bool ring = ring_len > 0 && ring_len % 4 == 0 && row_stride % 4 == 0;
+    if (status && aligned && (ring || ring_len == 0) && getenv("PV_DEDISP_V1") == nullptr) {
+        if (ring) a.stall = take_stall();
+        const int v = tma_tile(tdms, nout, ring_len, spread);
+        if (v >= 0) {
+            const int sp = spread(kTmaTiles[v].dms);
+            if (v == 0) return launch_dedisperse_tma<16, 32, 8, 2>(a, sp, status, s);
+            if (v == 1) return launch_dedisperse_tma<16, 32, 2, 4>(a, sp, status, s);
+            if (v == 2) return launch_dedisperse_tma<8, 32, 8, 2>(a, sp, status, s);
+            return launch_dedisperse_tma<8, 8, 16, 2>(a, sp, status, s);
+        }
     }
-    const int spread16 = delay_spread(h_dmshift, tdms, 16, start, step);
+    const int spread16 = spread(16);
     if ((size_t)2 * 4 * (1024 + spread16) * 4 <= 200 * 1024)
         return launch_dedisperse<16, 32, 4>(a, spread16, s);
-    const int spread8 = delay_spread(h_dmshift, tdms, 8, start, step);
+    const int spread8 = spread(8);
     if ((size_t)2 * 4 * (1024 + spread8) * 4 <= 220 * 1024)
         return launch_dedisperse<8, 32, 4>(a, spread8, s);
-    const int spread4 = delay_spread(h_dmshift, tdms, 4, start, step);
+    const int spread4 = spread(4);
     if ((size_t)2 * 2 * (512 + spread4) * 4 <= 220 * 1024)
         return launch_dedisperse<4, 16, 2>(a, spread4, s);
-    const int spread1 = delay_spread(h_dmshift, tdms, 1, start, step);
+    const int spread1 = spread(1);
     return launch_dedisperse<1, 16, 1>(a, spread1, s);
 }
 
@@ -1435,6 +1529,56 @@ extern "C" int pv_delay_table(int* d_shifts, const float* d_dmshift, int nchan, 
     return pv::check_launch("delay_table_kernel");
 }
 
+namespace {
+
+// Status words of pv_dedisperse_ex launches, one per call in turn, per device:
+// a call reports (and clears) what an earlier one recorded.
+constexpr int kExWords = 256;
+struct ExStatus {
+    int* words = nullptr;
+    unsigned next = 0;
+};
+std::mutex g_ex_mutex;
+std::map<int, ExStatus> g_ex;
+
+int ex_status(int** all, int** mine) {
+    int dev = 0;
+    PV_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
+    std::lock_guard<std::mutex> lk(g_ex_mutex);
+    ExStatus& e = g_ex[dev];
+    if (!e.words) {
+        PV_CUDA(cudaMalloc(&e.words, sizeof(int) * kExWords), "allocate dedispersion status");
+        PV_CUDA(cudaMemset(e.words, 0, sizeof(int) * kExWords), "clear dedispersion status");
+        PV_CUDA(cudaStreamSynchronize(cudaStreamLegacy), "clear dedispersion status");
+    }
+    *all = e.words;
+    *mine = e.words + e.next++ % kExWords;
+    return PV_OK;
+}
+
+// A thread's page-locked staging (reads from it need no copy by the driver).
+struct Staging {
+    void* p = nullptr;
+    size_t bytes = 0;
+    ~Staging() {
+        if (p) cudaFreeHost(p);
+    }
+    int get(size_t n, void** out) {
+        if (bytes < n) {
+            if (p) cudaFreeHost(p);
+            p = nullptr;
+            bytes = 0;
+            PV_CUDA(cudaHostAlloc(&p, n, cudaHostAllocPortable), "allocate staging");
+            bytes = n;
+        }
+        *out = p;
+        return PV_OK;
+    }
+};
+thread_local Staging t_staging;
+
+}  // namespace
+
 extern "C" int pv_dedisperse_ex(float* d_out, long long out_stride, const float* d_in,
                                 long long row_stride, long long row_len, int nchans, int nout,
                                 int tdms, const float* d_dmshift, float start_over_tsamp,
@@ -1447,9 +1591,22 @@ extern "C" int pv_dedisperse_ex(float* d_out, long long out_stride, const float*
     if (tdms == 0 || nout == 0) return PV_OK;
     std::vector<float> h(nchans);
     cudaStream_t s = pv::as_stream(stream);
-    PV_CUDA(cudaMemcpyAsync(h.data(), d_dmshift, sizeof(float) * nchans, cudaMemcpyDeviceToHost, s),
+    int *words = nullptr, *status = nullptr;
+    PV_TRY(ex_status(&words, &status));
+    void* staging = nullptr;
+    PV_TRY(t_staging.get(sizeof(float) * nchans + sizeof(int) * kExWords, &staging));
+    int* seen = reinterpret_cast<int*>(static_cast<float*>(staging) + nchans);
+    PV_CUDA(cudaMemcpyAsync(staging, d_dmshift, sizeof(float) * nchans, cudaMemcpyDeviceToHost, s),
             "copy dmshift");
+    PV_CUDA(cudaMemcpyAsync(seen, words, sizeof(int) * kExWords, cudaMemcpyDeviceToHost, s), "read status");
     PV_CUDA(cudaStreamSynchronize(s), "synchronise");
+    std::copy(static_cast<float*>(staging), static_cast<float*>(staging) + nchans, h.begin());
+    for (int i = 0; i < kExWords; ++i)
+        if (seen[i] != PV_OK) {
+            PV_CUDA(cudaMemsetAsync(words, 0, sizeof(int) * kExWords, s), "clear status");
+            pv::set_error("pv_dedisperse_ex: a pipeline wait of an earlier call gave up (status %d)", seen[i]);
+            return seen[i];
+        }
     // Every delay must be a finite, non-negative sample count: the tiles
     // address shared memory and the input relative to the first trial's delay.
     if (!(start_over_tsamp >= 0.0f) || !(step_over_tsamp >= 0.0f) ||
@@ -1471,8 +1628,10 @@ extern "C" int pv_dedisperse_ex(float* d_out, long long out_stride, const float*
             return PV_ERR_ARG;
         }
     }
-    return pv::dedisperse_device(d_out, out_stride, d_in, row_stride, row_len, 0, 0, nchans, nout,
-                                 tdms, d_dmshift, h, start_over_tsamp, step_over_tsamp, s, nullptr);
+    return pv::dedisperse_device(
+        d_out, out_stride, d_in, row_stride, row_len, 0, 0, nchans, nout, tdms, d_dmshift,
+        [&](int dms) { return delay_spread(h, tdms, dms, start_over_tsamp, step_over_tsamp); }, start_over_tsamp,
+        step_over_tsamp, s, status);
 }
 
 extern "C" int pv_dedisperse(float* d_out, long long out_bytes, const float* d_in,
@@ -1498,6 +1657,15 @@ struct pv_dedisp_plan {
     int* d_status = nullptr;  // PV_ERR_TIMEOUT if a pipeline wait gave up
     int nchan = 0, tdms = 0, max_shift = 0;
     float start = 0.0f, step = 0.0f;
+    // delay_spread by tile height, computed when first wanted (any thread)
+    mutable std::mutex spread_mutex;
+    mutable std::map<int, int> spreads;
+    int spread(int dms) const {
+        std::lock_guard<std::mutex> lk(spread_mutex);
+        auto it = spreads.find(dms);
+        if (it == spreads.end()) it = spreads.emplace(dms, delay_spread(h_dmshift, tdms, dms, start, step)).first;
+        return it->second;
+    }
 };
 
 extern "C" int pv_dedisp_plan_create(pv_dedisp_plan** plan, const float* h_dmshift, int nchans,
@@ -1587,6 +1755,6 @@ extern "C" int pv_dedisp_plan_run(const pv_dedisp_plan* p, float* d_out, long lo
     }
     if (nout == 0) return PV_OK;
     return pv::dedisperse_device(d_out, out_stride, d_in, row_stride, row_len, ring_len, t_base,
-                                 p->nchan, nout, p->tdms, p->d_dmshift, p->h_dmshift, p->start,
-                                 p->step, pv::as_stream(stream), p->d_status);
+                                 p->nchan, nout, p->tdms, p->d_dmshift, [p](int dms) { return p->spread(dms); },
+                                 p->start, p->step, pv::as_stream(stream), p->d_status);
 }

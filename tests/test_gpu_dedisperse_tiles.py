@@ -1,0 +1,90 @@
+"""The pipelined dedispersion's tiles on linear and ring rows against the
+oracle's FP32 sums, bit for bit: sizes around each tile's edges, delay spreads
+that only some tiles hold, rows at any stride, buffers at any alignment, and
+rows that end inside the spans (zeros beyond row_len, the next row where rows
+are contiguous, zeros beyond the buffer)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # nchan, tdms, nout, fch1, foff, DM step over tsamp
+    (40, 9, 255, 150.0, -0.05, 400.0),     # 8 x 256
+    (33, 17, 1025, 150.0, -0.05, 400.0),
+    (70, 300, 5003, 150.0, -0.05, 300.0),
+    (50, 600, 16500, 150.0, -0.05, 50.0),  # 16 x 1024
+    (24, 512, 10976, 150.0, -0.05, 100.0),  # 8 x 1024
+    (90, 40, 3000, 115.0, -0.05, 30000.0),  # spreads of thousands of samples
+]
+
+
+def _case(pv, oracle, case, seed=0):
+    nchan, tdms, nout, fch1, foff, step = case
+    k, _ = pv.dm_shifts(fch1, foff, nchan)
+    start, step = np.float32(1.5), np.float32(step)
+    ms = int(oracle.shift_table(k, tdms, start, step).max())
+    return k, start, step, ms, np.random.default_rng(seed + nchan)
+
+
+@pytest.mark.parametrize("case", CASES)
+@pytest.mark.parametrize("extra", [0, 1, 2, 3])
+def test_linear_rows(pv, oracle, cuda, case, extra):
+    import torch
+    nchan, tdms, nout = case[:3]
+    k, start, step, ms, rng = _case(pv, oracle, case)
+    width = nout + ms + extra  # extra 0: the last channel's last sample is the buffer's last
+    x = rng.standard_normal((nchan, width)).astype(np.float32)
+    want = oracle.dedisperse(x, nout, tdms, k, start, step)
+    kd = torch.from_numpy(k).to(cuda)
+    got = pv.dedisperse(torch.from_numpy(x).to(cuda), nout, tdms, kd, float(start), float(step))
+    assert np.array_equal(got.cpu().numpy(), want)
+    plan = pv.DedispPlan(k, tdms, float(start), float(step))
+    assert np.array_equal(plan.run(torch.from_numpy(x).to(cuda), nout).cpu().numpy(), want)
+    assert plan.status() == 0
+    if extra == 1:  # a buffer that is not 16-byte aligned
+        flat = torch.zeros(nchan * width + 1, device=cuda)
+        flat[1:] = torch.from_numpy(x.reshape(-1)).to(cuda)
+        got = pv.dedisperse(flat[1:].view(nchan, width), nout, tdms, kd, float(start), float(step))
+        assert np.array_equal(got.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("case", CASES[:3] + CASES[5:])
+@pytest.mark.parametrize("short", [1, 700])
+def test_rows_that_end_early(pv, oracle, cuda, case, short):
+    """row_len below what the delays reach: zeros beyond it; the same of a
+    contiguous buffer: the next row, and zeros beyond the last."""
+    import torch
+    nchan, tdms, nout = case[:3]
+    k, start, step, ms, rng = _case(pv, oracle, case, 1)
+    length = max(nout + ms - short, 1)
+    x = rng.standard_normal((nchan, length + 5)).astype(np.float32)
+    full = np.zeros((nchan, nout + ms + 1), np.float32)
+    full[:, :length] = x[:, :length]
+    want = oracle.dedisperse(full, nout, tdms, k, start, step)
+    kd = torch.from_numpy(k).to(cuda)
+    got = pv.dedisperse(torch.from_numpy(x).to(cuda), nout, tdms, kd, float(start), float(step), row_len=length)
+    assert np.array_equal(got.cpu().numpy(), want)
+    y = np.ascontiguousarray(x[:, :length])
+    flat = np.concatenate([y.reshape(-1), np.zeros(nout + ms + 1, np.float32)])
+    for c in range(nchan):
+        full[c] = flat[c * length:c * length + nout + ms + 1]
+    want = oracle.dedisperse(full, nout, tdms, k, start, step)
+    got = pv.dedisperse(torch.from_numpy(y).to(cuda), nout, tdms, kd, float(start), float(step))
+    assert np.array_equal(got.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_ring_rows(pv, oracle, cuda, case):
+    import torch
+    nchan, tdms, nout = case[:3]
+    k, start, step, ms, rng = _case(pv, oracle, case, 2)
+    ring = (nout + ms + 1100 + 3) // 4 * 4
+    lin = rng.standard_normal((nchan, ring)).astype(np.float32)
+    want = oracle.dedisperse(lin, nout, tdms, k, start, step)
+    plan = pv.DedispPlan(k, tdms, float(start), float(step))
+    for base in (0, ring - 5):
+        x = np.roll(lin, base, axis=1)
+        got = plan.run(torch.from_numpy(np.ascontiguousarray(x)).to(cuda), nout, ring_len=ring, t_base=base)
+        assert np.array_equal(got.cpu().numpy(), want)
+    assert plan.status() == 0

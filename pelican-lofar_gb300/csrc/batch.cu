@@ -100,7 +100,8 @@ struct pv_batch {
     struct ChanClass {
         int nchan = 0, njobs = 0;
         int packets = 0;  // the class's beams take LOFAR packets (one kernel per input layout)
-        long long nwarps = 0;
+        bool seg = false;
+        long long nunits = 0;  // warps (seg: CTAs)
         pv::ChanJob* d_jobs = nullptr;
     };
     std::vector<ChanClass> chan;
@@ -215,7 +216,7 @@ int enqueue_step(pv_batch* b, cudaStream_t s, bool capture) {
     PV_TRY(pv::check_launch("plan_kernel"));
     PV_TRY(mark(0, s));
     for (auto& c : b->chan)
-        PV_TRY(pv::launch_chan_fast(c.nchan, c.packets ? 2 : 1, c.d_jobs, pv::ChanJob{}, c.njobs, c.nwarps,
+        PV_TRY(pv::launch_chan_fast(c.nchan, c.packets ? 2 : 1, c.seg, c.d_jobs, pv::ChanJob{}, c.njobs, c.nunits,
                                     b->d_bs, s));
     PV_TRY(mark(1, s));
     // classes first..last-1 side by side, joined on s
@@ -419,14 +420,6 @@ extern "C" int pv_batch_create(pv_batch** out, const pv_beam_config* configs, in
         rc = pv::ppf_tables(x->ppf, &coeffs, &tw, &nchan, &ntaps);
         if (rc != PV_OK) return fail(rc);
         const int packets = x->cfg.udp_packet_bytes > 0 ? 1 : 0;
-        size_t k = 0;
-        while (k < b->chan.size() && (b->chan[k].nchan != nchan || b->chan[k].packets != packets)) ++k;
-        if (k == b->chan.size()) {
-            b->chan.emplace_back();
-            b->chan[k].nchan = nchan;
-            b->chan[k].packets = packets;
-            cj.emplace_back();
-        }
         pv::ChanJob j{};
         j.in = b->d_in[i];
         j.in_odd = b->d_in[nbeams + i];
@@ -442,8 +435,20 @@ extern "C" int pv_batch_create(pv_batch** out, const pv_beam_config* configs, in
         j.beam = i;
         j.pkt_bytes = x->cfg.udp_packet_bytes;
         j.pkt_nsub = x->cfg.udp_subbands;
-        j.warp_begin = b->chan[k].nwarps;
-        b->chan[k].nwarps += pv::chan_job_warps(j);
+        const bool seg = pv::chan_seg_supported(nchan, j);
+        size_t k = 0;
+        while (k < b->chan.size() &&
+               (b->chan[k].nchan != nchan || b->chan[k].packets != packets || b->chan[k].seg != seg))
+            ++k;
+        if (k == b->chan.size()) {
+            b->chan.emplace_back();
+            b->chan[k].nchan = nchan;
+            b->chan[k].packets = packets;
+            b->chan[k].seg = seg;
+            cj.emplace_back();
+        }
+        j.unit_begin = b->chan[k].nunits;
+        b->chan[k].nunits += pv::chan_job_units(j, nchan, seg, nbeams);
         cj[k].push_back(j);
     }
     for (size_t k = 0; k < b->chan.size(); ++k) {

@@ -331,12 +331,12 @@ chan_stokes_i_kernel(const pv::ChanJob* __restrict__ jobs, const __grid_constant
     int lo = 0, hi = njobs - 1;  // the job whose warps include gw
     while (jobs && lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (jobs[mid].warp_begin <= gw) lo = mid;
+        if (jobs[mid].unit_begin <= gw) lo = mid;
         else hi = mid - 1;
     }
     const pv::ChanJob& J = jobs ? jobs[lo] : one;
     const int nblocks = J.nblocks, window = J.window, nu = J.nu, nsub = J.nsub;
-    const long long local = gw - J.warp_begin;
+    const long long local = gw - J.unit_begin;
     const int s = (int)(local / J.nranges);
     const int r = (int)(local - (long long)s * J.nranges);
     const int B0 = r * kRangeBlocks;
@@ -499,6 +499,8 @@ chan_stokes_i_kernel(const pv::ChanJob* __restrict__ jobs, const __grid_constant
     }
 }
 
+#include "channelise_seg.cuh"
+
 // StokesGenerator::run on complex spectra [t][sub][2][N] (module-level call).
 __global__ void stokes_kernel(const float2* __restrict__ spectra, int nt, int nsub, int N, int nstokes,
                               float* __restrict__ out) {
@@ -607,14 +609,46 @@ bool chan_fast_supported(int nchan, int ntaps, int npol, int nstokes, int window
            nblocks >= kFastTaps - 1;
 }
 
-int chan_job_warps(ChanJob& job) {
-    job.nranges = ceil_div(job.nblocks, kRangeBlocks);
-    return job.nsub * job.nranges;
+bool chan_seg_supported(int nchan, const ChanJob& j) {
+    auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    return (nchan == 16 || nchan == 32) && j.pkt_bytes == 0 && j.window <= 8 && 8 % j.window == 0 &&
+           aligned(j.in) && aligned(j.in_odd) && aligned(j.out);
 }
 
-int launch_chan_fast(int nchan, int input, const ChanJob* d_jobs, const ChanJob& one, int njobs,
-                     long long nwarps, const BeamStep* bs, cudaStream_t s) {
-    if (nwarps <= 0) return PV_OK;
+long long chan_job_units(ChanJob& job, int nchan, bool seg, int parts) {
+    if (!seg) {
+        job.range = kRangeBlocks;
+        job.nranges = ceil_div(job.nblocks, kRangeBlocks);
+        return (long long)job.nsub * job.nranges;
+    }
+    // Every stream first reads the 7 blocks before its own: long streams where there are CTAs enough for
+    // the four of every SM, shorter ones (down to 32 blocks) where there are not.  4096 blocks of 32 x 16
+    // channels: 32.7 us in streams of 32 (128 CTAs), 38 of 128, 52 of 256; 65536 of 244: 831 of 256, 917 of 64.
+    const int streams = kSegThreads / nchan;
+    for (job.range = 256; job.range > 32; job.range /= 2)
+        if ((long long)job.nsub * ceil_div(job.nblocks, streams * job.range) * parts >= 4LL * sm_count()) break;
+    job.nranges = ceil_div(job.nblocks, streams * job.range);
+    return (long long)job.nsub * job.nranges;
+}
+
+int launch_chan_fast(int nchan, int input, bool seg, const ChanJob* d_jobs, const ChanJob& one, int njobs,
+                     long long nunits, const BeamStep* bs, cudaStream_t s) {
+    if (nunits <= 0) return PV_OK;
+    if (seg) {
+#define PV_CHAN_SEG(NN)                                                                                \
+    if (nchan == NN) {                                                                                 \
+        const unsigned g = (unsigned)nunits;                                                           \
+        if (input == 1) chan_stokes_seg_kernel<NN, true><<<g, kSegThreads, 0, s>>>(d_jobs, one, njobs, bs); \
+        else chan_stokes_seg_kernel<NN, false><<<g, kSegThreads, 0, s>>>(d_jobs, one, njobs, bs);      \
+        return check_launch("chan_stokes_seg_kernel");                                                 \
+    }
+        PV_CHAN_SEG(16)
+        PV_CHAN_SEG(32)
+#undef PV_CHAN_SEG
+        set_error("channelise: no segment kernel for %d channels", nchan);
+        return PV_ERR_ARG;
+    }
+    const long long nwarps = nunits;
     const unsigned grid = (unsigned)ceil_div<long long>(nwarps, 4);
 #define PV_CHAN_FAST(NN)                                                                         \
     if (nchan == NN) {                                                                           \
@@ -680,8 +714,9 @@ int run_channelise(pv_ppf* h, const void* d_in, int in_int16, int nsub, int npol
         job.nu = nu;
         job.pkt_bytes = pkt_bytes;
         job.pkt_nsub = pkt_nsub;
-        const long long nwarps = pv::chan_job_warps(job);
-        PV_TRY(pv::launch_chan_fast(h->nchan, pkt_bytes > 0 ? 2 : (in_int16 ? 1 : 0), nullptr, job, 1, nwarps,
+        const bool seg = pv::chan_seg_supported(h->nchan, job);
+        const long long units = pv::chan_job_units(job, h->nchan, seg, 1);
+        PV_TRY(pv::launch_chan_fast(h->nchan, pkt_bytes > 0 ? 2 : (in_int16 ? 1 : 0), seg, nullptr, job, 1, units,
                                     nullptr, s));
         h->cur ^= 1;
         h->have_hist = true;

@@ -35,8 +35,9 @@ struct ChanJob {
     const float* coeffs;     // [8][N]
     const float2* twiddle;   // [N/2] exp(-2 pi i k / N)
     float* out;              // [nu][sub][N] Stokes I
-    long long warp_begin;    // first warp of this job in the launch
+    long long unit_begin;    // first warp of this job in the launch (chan_stokes_seg_kernel: first CTA)
     int nsub, nblocks, window, nu, nranges;
+    int range;               // blocks of a stream (chan_stokes_seg_kernel)
     int beam;                // index into the batch's BeamStep array
     long long pkt_bytes;     // > 0: `in` holds LOFAR packets of this size (int16, 16 samples each)
     int pkt_nsub;            // subbands per packet; the nsub/pkt_nsub streams follow each other
@@ -46,11 +47,15 @@ bool chan_fast_supported(int nchan, int ntaps, int npol, int nstokes, int window
 // pkt_bytes > 0 (the register channeliser only)
 int channelise_stokes_i(pv_ppf* h, const void* d_in, int nsub, int nblocks, int window, int bin, float* d_stokes,
                         int* nu_out, long long pkt_bytes, int pkt_nsub, cudaStream_t s);
-int chan_job_warps(ChanJob& job);  // sets nranges, returns the job's warp count
+// chan_stokes_seg_kernel takes the job (voltages, not packets; N channels)
+bool chan_seg_supported(int nchan, const ChanJob& job);
+// Sets range and nranges for `parts` such jobs side by side in one launch; returns the job's warps
+// (seg: CTAs).
+long long chan_job_units(ChanJob& job, int nchan, bool seg, int parts);
 // bs == null: one job, always active, input `in`, history hist[0] -> hist[1].
 // input: 0 complex float voltages, 1 int16 voltages, 2 int16 LOFAR packets (pkt_bytes of every job)
-int launch_chan_fast(int nchan, int input, const ChanJob* d_jobs, const ChanJob& one, int njobs,
-                     long long nwarps, const BeamStep* bs, cudaStream_t s);
+int launch_chan_fast(int nchan, int input, bool seg, const ChanJob* d_jobs, const ChanJob& one, int njobs,
+                     long long nunits, const BeamStep* bs, cudaStream_t s);
 // Saved state of one beam (pv_beam_state_*): the PPF tap history and the
 // clipper's running state, as bytes in host memory.
 long long ppf_state_bytes(const pv_ppf* h, int nsub, int npol);

@@ -66,9 +66,16 @@ __device__ __forceinline__ float2 dif_upper(float2 u, float2 v, float2 w) {
 }
 __device__ __forceinline__ float2 times_minus_i(float2 d) { return make_float2(d.y, -d.x); }
 
-__global__ void __launch_bounds__(256) channelise_kernel(const ChanArgs a) {
+// POW2: N is a power of two (indices by shifts; BT always is one).  TT: the
+// number of taps where it is the usual 8 (the FIR unrolled), else 0.  Bound by
+// shared-memory accesses and issue: two FFT stages per pass, no divisions and
+// as many warps as the tile's shared memory leaves idle otherwise took 61
+// subbands x 64 channels x 4096 blocks from 838 to 438 us (spectra), 1041 to
+// 535 (four Stokes, x4).
+template <bool POW2, int TT>
+__global__ void __launch_bounds__(1024) channelise_kernel(const ChanArgs a) {
     extern __shared__ float2 sm[];
-    const int N = a.N, T = a.T, BT = a.BT, P = a.npol;
+    const int N = a.N, T = TT > 0 ? TT : a.T, BT = a.BT, P = a.npol;
     const int s = blockIdx.y;
     const int b0 = blockIdx.x * BT;
     const int nb = min(BT, a.nblocks - b0);  // blocks of this tile
@@ -77,65 +84,68 @@ __global__ void __launch_bounds__(256) channelise_kernel(const ChanArgs a) {
     float2* x = sm;                          // [P][BT+H][N]
     float2* y = sm + (size_t)P * (BT + H) * N;    // [P][BT][N]
     float2* tw = y + (size_t)P * BT * N;          // [N/2], or [N] for the direct DFT
-    const int ntw = a.log2n < 0 ? N : N / 2;
+    const int ntw = POW2 ? N / 2 : N;
     float* cf = reinterpret_cast<float*>(tw + N);  // [T][N]
     const int tid = threadIdx.x, nt = blockDim.x;
+    const int lg = a.log2n, lgb = __ffs(BT) - 1;
+    // i = row * N + c; and, of rows p * BT + b, the polarisation and block (b >= nb: none)
+    auto split = [&](int i, int& row, int& c) {
+        if (POW2) { row = i >> lg; c = i & (N - 1); }
+        else { row = i / N; c = i - row * N; }
+    };
 
     for (int i = tid; i < ntw; i += nt) tw[i] = a.twiddle[i];
     for (int i = tid; i < T * N; i += nt) cf[i] = a.coeffs[i];
     // stage blocks b0-H .. b0+nb-1; negative blocks come from the history
     for (int p = 0; p < P; ++p) {
-        const long long base = ((long long)s * P + p) * (long long)a.nblocks * N;
-        for (int i = tid; i < rows * N; i += nt) {
-            const int r = i / N, c = i - r * N;
-            const int b = b0 - H + r;
-            float2 v;
-            if (b >= 0) {
-                v = load_sample(a, base + (long long)b * N + c);
-            } else {
-                v = a.hist_in ? a.hist_in[(((long long)s * P + p) * H + (H + b)) * N + c]
-                              : make_float2(0.0f, 0.0f);
-            }
-            x[((size_t)p * (BT + H) + r) * N + c] = v;
+        const long long base = ((long long)s * P + p) * (long long)a.nblocks * N + (long long)(b0 - H) * N;
+        float2* xp = x + (size_t)p * (BT + H) * N;
+        const int past = b0 >= H ? 0 : (H - b0) * N;  // samples before the call's first block
+        if (past > 0) {
+            const float2* hist = a.hist_in ? a.hist_in + ((long long)s * P + p) * H * N + (long long)b0 * N : nullptr;
+            for (int i = tid; i < past; i += nt) xp[i] = hist ? hist[i] : make_float2(0.0f, 0.0f);
         }
+#pragma unroll 4
+        for (int i = past + tid; i < rows * N; i += nt) xp[i] = load_sample(a, base + i);
     }
     __syncthreads();
     // the last tile carries its final T-1 blocks (old history included when
     // the chunk is shorter than that) to the next call
     if (b0 + nb == a.nblocks && a.hist_out) {
         for (int p = 0; p < P; ++p)
-            for (int i = tid; i < H * N; i += nt) {
-                const int r = i / N, c = i - r * N;
-                a.hist_out[(((long long)s * P + p) * H + r) * N + c] =
-                    x[((size_t)p * (BT + H) + nb + r) * N + c];
-            }
+            for (int i = tid; i < H * N; i += nt)
+                a.hist_out[((long long)s * P + p) * H * N + i] = x[((size_t)p * (BT + H) + nb) * N + i];
     }
     // FIR: y[p][b][c] = sum_t coeff[t][c] * x[p][b+t][c], oldest tap first
-    for (int i = tid; i < P * nb * N; i += nt) {
-        const int c = i % N, pb = i / N;
-        const int p = pb / nb, b = pb - p * nb;
+    for (int i = tid; i < P * BT * N; i += nt) {
+        int row, c;
+        split(i, row, c);
+        const int p = row >> lgb, b = row & (BT - 1);
+        if (b >= nb) continue;
         const float2* xs = x + ((size_t)p * (BT + H) + b) * N + c;
         if (N == 1) {  // PPFChanneliser.cpp:108-131: one channel is the time series itself
-            y[(size_t)p * BT + b] = xs[(size_t)H * N];
+            y[i] = xs[(size_t)H * N];
             continue;
         }
         float re = 0.0f, im = 0.0f;
-        for (int t = 0; t < T; ++t) {
+#pragma unroll
+        for (int t = 0; t < (TT > 0 ? TT : T); ++t) {
             const float k = cf[t * N + c];
             const float2 v = xs[(size_t)t * N];
             re = __fmaf_rn(v.x, k, re);
             im = __fmaf_rn(v.y, k, im);
         }
-        y[((size_t)p * BT + b) * N + c] = make_float2(re, im);
+        y[i] = make_float2(re, im);
     }
     __syncthreads();
-    if (a.log2n < 0) {
+    if (!POW2) {
         // N not a power of two: the forward DFT sum_j y[j] exp(-2 pi i j k / N) of every row
         // into x (no longer needed), in natural channel order
-        for (int i = tid; i < P * nb * N; i += nt) {
-            const int k = i % N, pb = i / N;
-            const int p = pb / nb, b = pb - p * nb;
-            const float2* r = y + ((size_t)p * BT + b) * N;
+        for (int i = tid; i < P * BT * N; i += nt) {
+            int row, k;
+            split(i, row, k);
+            if ((row & (BT - 1)) >= nb) continue;
+            const float2* r = y + (size_t)row * N;
             float re = 0.0f, im = 0.0f;
             int m = 0;  // j * k mod N
             for (int j = 0; j < N; ++j) {
@@ -145,27 +155,47 @@ __global__ void __launch_bounds__(256) channelise_kernel(const ChanArgs a) {
                 m += k;
                 if (m >= N) m -= N;
             }
-            x[((size_t)p * BT + b) * N + k] = make_float2(re, im);
+            x[i] = make_float2(re, im);
         }
         __syncthreads();
     }
     // In-place radix-2 decimation-in-frequency FFT of every (pol, block) row
-    // of y (dif_upper gives the butterfly arithmetic); row position i then
-    // holds channel bitrev(i).
-    const int half = N / 2, lg = a.log2n;
-    for (int lh = lg - 1; lh >= 0; --lh) {  // no stage when lg <= 0
-        const int h = 1 << lh;
-        for (int i = tid; i < P * nb * half; i += nt) {
-            const int j = i & (half - 1), row = i >> (lg - 1);
-            const int p = row / nb, b = row - p * nb;
-            float2* r = y + ((size_t)p * BT + b) * N;
-            const int lo = ((j >> lh) << (lh + 1)) + (j & (h - 1));
-            const float2 u = r[lo], v = r[lo + h];
-            r[lo] = make_float2(__fadd_rn(u.x, v.x), __fadd_rn(u.y, v.y));
-            const float2 d = make_float2(__fsub_rn(u.x, v.x), __fsub_rn(u.y, v.y));
-            if (lh == 0) r[lo + h] = d;                                   // twiddle 1
-            else if (lh == 1) r[lo + h] = (j & 1) ? times_minus_i(d) : d;  // 1 or -i
-            else r[lo + h] = twiddle_mul(d, tw[(j & (h - 1)) << (lg - 1 - lh)]);
+    // of y (dif_upper gives the butterfly arithmetic), two stages per pass
+    // where two are left; row position i then holds channel bitrev(i).
+    auto upper = [&](float2 d, int lh, int q) {  // the upper output of a butterfly of span 2^lh at q
+        if (lh == 0) return d;                                  // twiddle 1
+        if (lh == 1) return (q & 1) ? times_minus_i(d) : d;     // 1 or -i
+        return twiddle_mul(d, tw[q << (lg - 1 - lh)]);
+    };
+    auto sum = [](float2 u, float2 v) { return make_float2(__fadd_rn(u.x, v.x), __fadd_rn(u.y, v.y)); };
+    auto diff = [](float2 u, float2 v) { return make_float2(__fsub_rn(u.x, v.x), __fsub_rn(u.y, v.y)); };
+    int lh = lg - 1;  // no stage when lg <= 0
+    for (; lh >= 1; lh -= 2) {
+        const int h = 1 << lh, g = h >> 1, quarter = N / 4;
+        for (int i = tid; i < P * BT * quarter; i += nt) {
+            const int row = i >> (lg - 2), j = i & (quarter - 1);
+            if ((row & (BT - 1)) >= nb) continue;
+            const int q = j & (g - 1);
+            float2* r = y + (size_t)row * N + ((j >> (lh - 1)) << (lh + 1)) + q;
+            const float2 v0 = r[0], v1 = r[g], v2 = r[h], v3 = r[h + g];
+            const float2 a0 = sum(v0, v2), a1 = sum(v1, v3);
+            const float2 a2 = upper(diff(v0, v2), lh, q), a3 = upper(diff(v1, v3), lh, q + g);
+            r[0] = sum(a0, a1);
+            r[g] = upper(diff(a0, a1), lh - 1, q);
+            r[h] = sum(a2, a3);
+            r[h + g] = upper(diff(a2, a3), lh - 1, q);
+        }
+        __syncthreads();
+    }
+    if (lh == 0) {
+        const int half = N / 2;
+        for (int i = tid; i < P * BT * half; i += nt) {
+            const int row = i >> (lg - 1), j = i & (half - 1);
+            if ((row & (BT - 1)) >= nb) continue;
+            float2* r = y + (size_t)row * N + 2 * j;
+            const float2 u = r[0], v = r[1];
+            r[0] = sum(u, v);
+            r[1] = diff(u, v);
         }
         __syncthreads();
     }
@@ -174,11 +204,12 @@ __global__ void __launch_bounds__(256) channelise_kernel(const ChanArgs a) {
     auto pos = [lg](int c) { return lg > 0 ? (int)(__brev((unsigned)c) >> (32 - lg)) : c; };
     // src holds the spectra, rows of stride N with pol stride BT*N
     if (a.mode == 0) {
-        for (int i = tid; i < P * nb * N; i += nt) {
-            const int c = i % N, pb = i / N;
-            const int b = pb % nb, p = pb / nb;
-            a.spectra[(((long long)(b0 + b) * a.nsub + s) * P + p) * N + c] =
-                src[((size_t)p * BT + b) * N + pos(c)];
+        for (int i = tid; i < P * BT * N; i += nt) {
+            int row, c;
+            split(i, row, c);
+            const int p = row >> lgb, b = row & (BT - 1);
+            if (b < nb)
+                a.spectra[(((long long)(b0 + b) * a.nsub + s) * P + p) * N + c] = src[(size_t)row * N + pos(c)];
         }
         return;
     }
@@ -548,6 +579,28 @@ __global__ void integrate_kernel(const float* __restrict__ in, int nsub, int npo
     }
 }
 
+// The same without channel binning, four adjacent values of the n of a
+// spectrum (every subband, polarisation and channel) per thread: the loads of
+// several spectra are in flight while their sums are added in order.  65 MB of
+// 2050 x 62 x 4 x 32 values over 16 spectra: 31 us against 54, call included.
+__global__ void integrate4_kernel(const float4* __restrict__ in, long long n4, int window, int nu,
+                                  float4* __restrict__ out) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= n4 * nu) return;
+    const long long u = i / n4;
+    const float4* v = in + u * window * n4 + (i - u * n4);
+    float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 8
+    for (int t = 0; t < window; ++t) {
+        const float4 x = __ldcs(v + t * n4);
+        a.x = __fadd_rn(a.x, x.x);
+        a.y = __fadd_rn(a.y, x.y);
+        a.z = __fadd_rn(a.z, x.z);
+        a.w = __fadd_rn(a.w, x.w);
+    }
+    out[i] = a;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -638,8 +691,12 @@ int launch_chan_fast(int nchan, int input, bool seg, const ChanJob* d_jobs, cons
 #define PV_CHAN_SEG(NN)                                                                                \
     if (nchan == NN) {                                                                                 \
         const unsigned g = (unsigned)nunits;                                                           \
-        if (input == 1) chan_stokes_seg_kernel<NN, true><<<g, kSegThreads, 0, s>>>(d_jobs, one, njobs, bs); \
-        else chan_stokes_seg_kernel<NN, false><<<g, kSegThreads, 0, s>>>(d_jobs, one, njobs, bs);      \
+        if (input == 3)                                                                                \
+            chan_stokes_seg_kernel<NN, false, true><<<g, kSegThreads, 0, s>>>(d_jobs, one, njobs, bs); \
+        else if (input == 1)                                                                           \
+            chan_stokes_seg_kernel<NN, true, false><<<g, kSegThreads, 0, s>>>(d_jobs, one, njobs, bs); \
+        else                                                                                           \
+            chan_stokes_seg_kernel<NN, false, false><<<g, kSegThreads, 0, s>>>(d_jobs, one, njobs, bs); \
         return check_launch("chan_stokes_seg_kernel");                                                 \
     }
         PV_CHAN_SEG(16)
@@ -700,24 +757,28 @@ int run_channelise(pv_ppf* h, const void* d_in, int in_int16, int nsub, int npol
         pv::set_error("channelise: packet input needs int16 samples, 16/32/64 channels, 8 taps, Stokes I");
         return PV_ERR_ARG;
     }
-    if (fast && (pkt_bytes > 0 || getenv("PV_CHAN_GENERIC") == nullptr)) {
+    // complex spectra of two polarisations: the two-phase kernel as well
+    const bool spectra = mode == 0 && npol == 2 && !in_int16 && h->ntaps == kFastTaps && nblocks >= kFastTaps - 1 &&
+                         (h->nchan == 16 || h->nchan == 32) && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0 &&
+                         (reinterpret_cast<uintptr_t>(d_spectra) & 15) == 0;
+    if ((fast || spectra) && (pkt_bytes > 0 || getenv("PV_CHAN_GENERIC") == nullptr)) {
         pv::ChanJob job{};
         job.in = d_in;
         job.hist[0] = h->have_hist ? h->d_hist[h->cur] : nullptr;
         job.hist[1] = h->d_hist[h->cur ^ 1];
         job.coeffs = h->d_coeffs;
         job.twiddle = h->d_twiddle;
-        job.out = d_stokes;
+        job.out = spectra ? reinterpret_cast<float*>(d_spectra) : d_stokes;
         job.nsub = nsub;
         job.nblocks = nblocks;
         job.window = w;
         job.nu = nu;
         job.pkt_bytes = pkt_bytes;
         job.pkt_nsub = pkt_nsub;
-        const bool seg = pv::chan_seg_supported(h->nchan, job);
+        const bool seg = spectra || pv::chan_seg_supported(h->nchan, job);
         const long long units = pv::chan_job_units(job, h->nchan, seg, 1);
-        PV_TRY(pv::launch_chan_fast(h->nchan, pkt_bytes > 0 ? 2 : (in_int16 ? 1 : 0), seg, nullptr, job, 1, units,
-                                    nullptr, s));
+        PV_TRY(pv::launch_chan_fast(h->nchan, spectra ? 3 : (pkt_bytes > 0 ? 2 : (in_int16 ? 1 : 0)), seg, nullptr,
+                                    job, 1, units, nullptr, s));
         h->cur ^= 1;
         h->have_hist = true;
         if (nu_out) *nu_out = nu;
@@ -734,15 +795,22 @@ int run_channelise(pv_ppf* h, const void* d_in, int in_int16, int nsub, int npol
     a.N = h->nchan; a.T = h->ntaps; a.log2n = h->log2n; a.BT = bt;
     a.mode = mode; a.spectra = d_spectra; a.stokes = d_stokes;
     a.nstokes = nstokes; a.window = w; a.bin = bin; a.nu = nu;
-    PV_CUDA(cudaFuncSetAttribute(channelise_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem), "cudaFuncSetAttribute(channelise)");
+    // warps for the shared memory that a CTA takes from the SM
+    const int threads = smem > 110 * 1024 ? 1024 : (smem > 72 * 1024 ? 512 : 256);
     dim3 grid((unsigned)pv::ceil_div(nblocks, bt), (unsigned)nsub);
     if (nsub > 65535) {
         pv::set_error("channelise: too many subbands");
         return PV_ERR_ARG;
     }
-    channelise_kernel<<<grid, 256, smem, s>>>(a);
-    PV_TRY(pv::check_launch("channelise_kernel"));
+    auto launch = [&](auto kern) -> int {
+        PV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                "cudaFuncSetAttribute(channelise)");
+        kern<<<grid, threads, smem, s>>>(a);
+        return pv::check_launch("channelise_kernel");
+    };
+    if (h->log2n < 0) PV_TRY(launch(channelise_kernel<false, 0>));
+    else if (h->ntaps == 8) PV_TRY(launch(channelise_kernel<true, 8>));
+    else PV_TRY(launch(channelise_kernel<true, 0>));
     if (h->ntaps > 1) {
         h->cur ^= 1;
         h->have_hist = true;
@@ -911,6 +979,13 @@ extern "C" int pv_integrate(const float* d_in, int nt, int nsub, int npol, int n
     if (nu_out) *nu_out = nu;
     const long long n = (long long)nu * nsub * npol * (nchan / bin);
     if (n == 0) return PV_OK;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(d_in) | reinterpret_cast<uintptr_t>(d_out)) & 15) == 0;
+    const long long spectrum = (long long)nsub * npol * nchan;
+    if (bin == 1 && spectrum % 4 == 0 && aligned && n / 4 <= 256LL * 0x7fffffff) {
+        integrate4_kernel<<<(unsigned)pv::ceil_div<long long>(n / 4, 256), 256, 0, pv::as_stream(stream)>>>(
+            reinterpret_cast<const float4*>(d_in), spectrum / 4, w, nu, reinterpret_cast<float4*>(d_out));
+        return pv::check_launch("integrate4_kernel");
+    }
     const int blocks = (int)std::min<long long>(pv::ceil_div<long long>(n, 256), pv::sm_count() * 16LL);
     integrate_kernel<<<blocks, 256, 0, pv::as_stream(stream)>>>(d_in, nsub, npol, nchan, w, bin, nu,
                                                                d_out);

@@ -1,7 +1,7 @@
 // K1 fast path in two phases through shared memory (included by channelise.cu
 // inside its anonymous namespace, after FirWindow): Stokes I of a
 // dual-polarisation, 8-tap PPF with N = 16 or 32 channels, integrated over 1,
-// 2, 4 or 8 blocks.
+// 2, 4 or 8 blocks; or its complex spectra.
 //
 // A CTA of 128 threads takes one subband and 128/N streams of `range`
 // consecutive blocks each, 8 blocks of every stream per phase:
@@ -42,8 +42,10 @@ __device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigne
 }
 
 // 16-point decimation-in-frequency FFT, output in bit-reversed places.  The
-// twiddles exp(-2 pi i e / 16) to FP32 are the table's values; the products
-// with 1 and -i, exact in twiddle_mul, are left out.
+// twiddles exp(-2 pi i e / 16) to FP32 are the table's values.  Products with 1
+// and -i are exact and left out, but for FULL (float voltages, which may be
+// infinite: the product's infinity times 0 is then part of the result).
+template <bool FULL>
 struct Fft16 {
     unsigned long long v[16];
     template <int H>
@@ -55,14 +57,16 @@ struct Fft16 {
             const unsigned long long a = v[lo], b = v[lo + H];
             v[lo] = add2(a, b);
             const unsigned long long d = sub2(a, b);
-            if (e == 0) {
+            if (e == 0 && !(FULL && H >= 4)) {
                 v[lo + H] = d;
-            } else if (e == 4) {
+            } else if (e == 4 && !(FULL && H >= 4)) {
                 const float2 z = times_minus_i(upk2(d));
                 v[lo + H] = pk2(z.x, z.y);
             } else {
                 constexpr float c1 = 0x1.d906bcp-1f, c2 = 0x1.6a09e6p-1f, c3 = 0x1.87de2ap-2f;
-                const float2 w = e == 1   ? make_float2(c1, -c3)
+                const float2 w = e == 0   ? make_float2(1.0f, -0.0f)
+                                 : e == 4 ? make_float2(0.0f, -1.0f)
+                                 : e == 1 ? make_float2(c1, -c3)
                                  : e == 2 ? make_float2(c2, -c2)
                                  : e == 3 ? make_float2(c3, -c1)
                                  : e == 5 ? make_float2(-c3, -c1)
@@ -80,6 +84,27 @@ struct Fft16 {
             v[2 * k] = x.x;
             v[2 * k + 1] = x.y;
         }
+    }
+    // Channels in order: row of 16 * M, this being segment k of M.
+    template <int M>
+    __device__ __forceinline__ void store(float* row, int k) const {
+        if constexpr (M == 1) {
+#pragma unroll
+            for (int c = 0; c < 16; c += 2) {
+                ulonglong2 x;
+                x.x = v[brev4(c)];
+                x.y = v[brev4(c + 1)];
+                *reinterpret_cast<ulonglong2*>(row + 2 * c) = x;
+            }
+        } else {
+            __syncwarp();  // the row's other segment has been read
+#pragma unroll
+            for (int c = 0; c < 16; ++c)
+                *reinterpret_cast<unsigned long long*>(row + 2 * (M * c + k)) = v[brev4(c)];
+        }
+    }
+    static constexpr __device__ int brev4(int c) {
+        return (c & 1) << 3 | (c & 2) << 1 | (c & 4) >> 1 | (c & 8) >> 3;
     }
     __device__ __forceinline__ void run() {
         stage<8>();
@@ -117,7 +142,8 @@ struct SegRaw {
     __device__ __forceinline__ float2 get(int k) const { return RawSample<I16>::f2(x[k]); }
 };
 
-template <int N, bool I16>
+// SPECTRA: J.out takes the complex spectra [block][sub][pol][N] instead.
+template <int N, bool I16, bool SPECTRA>
 __global__ void __launch_bounds__(kSegThreads, 4)
 chan_stokes_seg_kernel(const pv::ChanJob* __restrict__ jobs, const __grid_constant__ pv::ChanJob one, int njobs,
                        const pv::BeamStep* __restrict__ bs) {
@@ -213,11 +239,30 @@ chan_stokes_seg_kernel(const pv::ChanJob* __restrict__ jobs, const __grid_consta
         }
         __syncthreads();
         const int seg0 = (tid >> 5) * 16;  // the warp's first segment
+        // the warp's rows of N spectrum values, 16 bytes per lane
+        auto copy_spectra = [&]() {
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+                const int sl = it * 4 + (lane >> 3), q = sl >> 4, sg = seg0 + (sl & 15);
+                const int lb = sg / M, k = sg % M, at = k * 32 + (lane & 7) * 4;  // words into the row
+                const int b = first + (lb >> 3) * range + p0 + (lb & 7);
+                const float4 x = *reinterpret_cast<const float4*>(sm + q * POL + lb * M * kSegWords + at);
+                if (b < nblocks)
+                    *reinterpret_cast<float4*>(J.out + (((long long)b * nsub + s) * 2 + q) * 2 * N + at) = x;
+            }
+        };
         {
             float* seg = sm + (lane >> 4) * POL + (seg0 + (lane & 15)) * kSegWords;
-            Fft16 f;
+            Fft16<!I16> f;
             f.load(seg);
             f.run();
+            if constexpr (SPECTRA) {
+                f.template store<M>(sm + (lane >> 4) * POL + (seg0 + (lane & 15)) / M * (M * kSegWords), (lane & 15) % M);
+                __syncwarp();
+                copy_spectra();
+                __syncthreads();
+                continue;
+            }
             float p[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) p[i] = f.power(i);

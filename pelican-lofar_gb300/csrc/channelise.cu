@@ -663,9 +663,9 @@ bool chan_fast_supported(int nchan, int ntaps, int npol, int nstokes, int window
 }
 
 bool chan_seg_supported(int nchan, const ChanJob& j) {
-    auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    return (nchan == 16 || nchan == 32) && j.pkt_bytes == 0 && j.window <= 8 && 8 % j.window == 0 &&
-           aligned(j.in) && aligned(j.in_odd) && aligned(j.out);
+    auto aligned = [&](const void* p) { return j.pkt_bytes > 0 || (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    return (nchan == 16 || nchan == 32 || nchan == 64) && j.window <= 8 && 8 % j.window == 0 && aligned(j.in) &&
+           aligned(j.in_odd);
 }
 
 long long chan_job_units(ChanJob& job, int nchan, bool seg, int parts) {
@@ -675,11 +675,15 @@ long long chan_job_units(ChanJob& job, int nchan, bool seg, int parts) {
         return (long long)job.nsub * job.nranges;
     }
     // Every stream first reads the 7 blocks before its own: long streams where there are CTAs enough for
-    // the four of every SM, shorter ones (down to 32 blocks) where there are not.  4096 blocks of 32 x 16
-    // channels: 32.7 us in streams of 32 (128 CTAs), 38 of 128, 52 of 256; 65536 of 244: 831 of 256, 917 of 64.
-    const int streams = kSegThreads / nchan;
-    for (job.range = 256; job.range > 32; job.range /= 2)
-        if ((long long)job.nsub * ceil_div(job.nblocks, streams * job.range) * parts >= 4LL * sm_count()) break;
+    // some rounds over the SMs (4 resident on each, 2 for 64 channels), shorter ones where there are not.  4096
+    // blocks of 32 x 16 channels: 32 us in streams of 32 (128 CTAs), 39 of 128, 52 of 256; 65536 of 244 x 16:
+    // 833 us of 256, 920 of 64; 16391 of 61 x 64: 287 us of 128 (6.6 rounds), 297 of 256 (3.4).
+    const int streams = nchan == 64 ? 4 : kSegThreads / nchan;
+    const long long round = (nchan == 64 ? 2LL : 4LL) * sm_count();
+    auto ctas = [&](int range) { return (long long)job.nsub * ceil_div(job.nblocks, streams * range) * parts; };
+    job.range = 256;
+    while (job.range > 64 && ctas(job.range) < (nchan == 64 ? 5 : 3) * round) job.range /= 2;
+    if (ctas(job.range) < round) job.range = 32;
     job.nranges = ceil_div(job.nblocks, streams * job.range);
     return (long long)job.nsub * job.nranges;
 }
@@ -688,22 +692,25 @@ int launch_chan_fast(int nchan, int input, bool seg, const ChanJob* d_jobs, cons
                      long long nunits, const BeamStep* bs, cudaStream_t s) {
     if (nunits <= 0) return PV_OK;
     if (seg) {
-#define PV_CHAN_SEG(NN)                                                                                \
-    if (nchan == NN) {                                                                                 \
-        const unsigned g = (unsigned)nunits;                                                           \
-        if (input == 3)                                                                                \
-            chan_stokes_seg_kernel<NN, false, true><<<g, kSegThreads, 0, s>>>(d_jobs, one, njobs, bs); \
-        else if (input == 1)                                                                           \
-            chan_stokes_seg_kernel<NN, true, false><<<g, kSegThreads, 0, s>>>(d_jobs, one, njobs, bs); \
-        else                                                                                           \
-            chan_stokes_seg_kernel<NN, false, false><<<g, kSegThreads, 0, s>>>(d_jobs, one, njobs, bs); \
-        return check_launch("chan_stokes_seg_kernel");                                                 \
+        const unsigned g = (unsigned)nunits;
+#define PV_CHAN_SEG(NN, I16, PKT, SPECTRA) \
+    if (nchan == NN) chan_stokes_seg_kernel<NN, I16, PKT, SPECTRA><<<g, kSegThreads, 0, s>>>(d_jobs, one, njobs, bs);
+#define PV_CHAN_SEGS(IN, I16, PKT)        \
+    if (input == IN) {                    \
+        PV_CHAN_SEG(16, I16, PKT, false)  \
+        PV_CHAN_SEG(32, I16, PKT, false)  \
+        PV_CHAN_SEG(64, I16, PKT, false)  \
     }
-        PV_CHAN_SEG(16)
-        PV_CHAN_SEG(32)
+        PV_CHAN_SEGS(0, false, false)
+        PV_CHAN_SEGS(1, true, false)
+        PV_CHAN_SEGS(2, true, true)
+        if (input == 3) {
+            PV_CHAN_SEG(16, false, false, true)
+            PV_CHAN_SEG(32, false, false, true)
+        }
+        return check_launch("chan_stokes_seg_kernel");
+#undef PV_CHAN_SEGS
 #undef PV_CHAN_SEG
-        set_error("channelise: no segment kernel for %d channels", nchan);
-        return PV_ERR_ARG;
     }
     const long long nwarps = nunits;
     const unsigned grid = (unsigned)ceil_div<long long>(nwarps, 4);

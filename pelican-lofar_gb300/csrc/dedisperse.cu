@@ -20,6 +20,7 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include <cuda_fp16.h>
@@ -611,11 +612,16 @@ dedisperse_batch_kernel(const pv::DdJob* __restrict__ jobs, const pv::DdTile* __
     // funnel shift of two when the offset is not a multiple of 4; a byte q
     // stands for (q - 128) * scale + offset of its channel, the offsets of all
     // channels being added once per output.  When every row of the beam has
-    // the same scale, the codes themselves are summed exactly as integers:
-    // bytes 0 and 2 (1 and 3) of a word go to the two 16-bit halves of one
-    // register, which take 257 codes before a carry could cross, so the
-    // halves move into 32-bit sums every 256 channels; the output is then
-    // scale * (sum - 128 * nchan) + offset sum.
+    // the same scale, the codes themselves are summed exactly as integers, two
+    // channels at a time: bytes 1 and 3 of the words in the two 16-bit halves
+    // of one register, which take 257 codes before a carry could cross, and the
+    // words as they are (modulo 2^32) in another.  Every 256 channels the
+    // second less the first shifted up is the sum of bytes 0 and 2 in halves,
+    // and the halves move into 32-bit sums; the output is then scale * (sum -
+    // 128 * nchan) + offset sum.  Bound by the integer pipe: 2.75 operations
+    // per word (two three-operand adds and two byte permutes per two words, a
+    // funnel shift for three offsets of four) against 4.75 when bytes 0 and 2
+    // were spread as well (four beams of 244 to 61 subbands, 7.1 to 6.6 ms a step).
     unsigned gs = 0;
     for (;;) {
         const int b0 = gs % ST;
@@ -634,23 +640,38 @@ dedisperse_batch_kernel(const pv::DdJob* __restrict__ jobs, const pv::DdTile* __
         const int nchan = J.nchan;
         const int nst = (nchan + CS - 1) / CS;
         if (STORE == PV_STORE_U8 && J.uniform) {
-            unsigned pk[R / 2];  // [2q]: samples 4l, 4l+2 of group q; [2q+1]: 4l+1, 4l+3
+            unsigned all[R / 4], odd[R / 4];  // of group q: words; samples 4l+1 and 4l+3 in halves
             int isum[R];
 #pragma unroll
-            for (int r = 0; r < R / 2; ++r) pk[r] = 0u;
+            for (int q = 0; q < R / 4; ++q) all[q] = odd[q] = 0u;
 #pragma unroll
             for (int r = 0; r < R; ++r) isum[r] = 0;
             auto flush = [&]() {
 #pragma unroll
                 for (int q = 0; q < R / 4; ++q) {
-                    isum[4 * q + 0] += (int)(pk[2 * q] & 0xffffu);
-                    isum[4 * q + 2] += (int)(pk[2 * q] >> 16);
-                    isum[4 * q + 1] += (int)(pk[2 * q + 1] & 0xffffu);
-                    isum[4 * q + 3] += (int)(pk[2 * q + 1] >> 16);
-                    pk[2 * q] = 0u;
-                    pk[2 * q + 1] = 0u;
+                    const unsigned even = all[q] - (odd[q] << 8);  // samples 4l and 4l+2 in halves
+                    isum[4 * q + 0] += (int)(even & 0xffffu);
+                    isum[4 * q + 2] += (int)(even >> 16);
+                    isum[4 * q + 1] += (int)(odd[q] & 0xffffu);
+                    isum[4 * q + 3] += (int)(odd[q] >> 16);
+                    all[q] = odd[q] = 0u;
                 }
             };
+            // word q of a channel whose row offset is m bytes past a word
+            auto word = [](const unsigned* wr, int q, int m, bool shifted) {
+                const unsigned x = wr[32 * q];
+                return shifted ? __funnelshift_r(x, wr[32 * q + 1], 8 * m) : x;
+            };
+            auto add_two = [&](const unsigned* w0, int m0, const unsigned* w1, int m1, auto s0, auto s1) {
+#pragma unroll
+                for (int q = 0; q < R / 4; ++q) {
+                    const unsigned x = word(w0, q, m0, s0.value), y = word(w1, q, m1, s1.value);
+                    all[q] += x + y;
+                    odd[q] += __byte_perm(x, 0u, 0x4341u) + __byte_perm(y, 0u, 0x4341u);
+                }
+            };
+            using Yes = std::true_type;
+            using No = std::false_type;
             for (int st = 0; st < nst; ++st) {
                 const int b = gs % ST;
                 if (st > 0 && !mbar_wait_warp(&full[b], (gs / ST) & 1u, wait_ns)) {
@@ -662,17 +683,28 @@ dedisperse_batch_kernel(const pv::DdJob* __restrict__ jobs, const pv::DdTile* __
                     const int my_off =
                         lane < c_end ? min(pv_shift(meta_k[b * CS + lane], dv) - meta_off[b * CS + lane], slot - TT - 4)
                                      : 0;
-                    for (int j = 0; j < c_end; ++j) {
-                        const int off = __shfl_sync(0xffffffffu, my_off, j);
-                        const unsigned* wr =
-                            reinterpret_cast<const unsigned*>(slots + (size_t)(b * CS + j) * slot) + (off >> 2) + lane;
-                        const int m = off & 3;
+                    for (int j = 0; j < c_end; j += 2) {
+                        const int o0 = __shfl_sync(0xffffffffu, my_off, j);
+                        const int o1 = __shfl_sync(0xffffffffu, my_off, (j + 1) & 31);
+                        const unsigned* row = reinterpret_cast<const unsigned*>(slots + (size_t)(b * CS + j) * slot);
+                        const unsigned* w0 = row + (o0 >> 2) + lane;
+                        const int m0 = o0 & 3, m1 = o1 & 3;
+                        if (j + 1 == c_end) {  // an odd number of channels
 #pragma unroll
-                        for (int q = 0; q < R / 4; ++q) {
-                            unsigned x = wr[32 * q];
-                            if (m) x = __funnelshift_r(x, wr[32 * q + 1], 8 * m);
-                            pk[2 * q] += __byte_perm(x, 0u, 0x4240u);
-                            pk[2 * q + 1] += __byte_perm(x, 0u, 0x4341u);
+                            for (int q = 0; q < R / 4; ++q) {
+                                const unsigned x = word(w0, q, m0, m0 != 0);
+                                all[q] += x;
+                                odd[q] += __byte_perm(x, 0u, 0x4341u);
+                            }
+                            break;
+                        }
+                        const unsigned* w1 = row + (slot >> 2) + (o1 >> 2) + lane;  // slots are whole words
+                        if (m0) {
+                            if (m1) add_two(w0, m0, w1, m1, Yes{}, Yes{});
+                            else add_two(w0, m0, w1, m1, Yes{}, No{});
+                        } else {
+                            if (m1) add_two(w0, m0, w1, m1, No{}, Yes{});
+                            else add_two(w0, m0, w1, m1, No{}, No{});
                         }
                     }
                     if ((st + 1) % (256 / CS) == 0) flush();

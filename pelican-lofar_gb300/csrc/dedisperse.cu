@@ -220,8 +220,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
 // completion itself (acquire), and the give-up decision comes from lane 0's
 // clock, so the warp leaves the wait together.  Gives up after limit_ns.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, unsigned parity, unsigned long long limit_ns) {
+    bool done = mbar_try_wait(bar, parity);
+    if (__all_sync(0xffffffffu, done)) return true;
     const unsigned long long t_end = global_ns() + limit_ns;
-    bool done = false;
     for (;;) {
         if (!done) done = mbar_try_wait(bar, parity);
         if (__all_sync(0xffffffffu, done)) return true;
@@ -235,127 +236,155 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
         ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
+// Shared memory of a pipelined launch: slots [ST * CS][slot], per channel the
+// row offset and delay constant, the barriers.
+template <int CS, int ST>
+struct Pipe {
+    float* slots;
+    int* meta_off;
+    float* meta_k;
+    uint64_t *full, *empty;
+    __device__ __forceinline__ Pipe(unsigned char* smem, int slot) {
+        slots = reinterpret_cast<float*>(smem);
+        meta_off = reinterpret_cast<int*>(slots + (size_t)ST * CS * slot);
+        meta_k = reinterpret_cast<float*>(meta_off + ST * CS);
+        // slot is a multiple of 4 floats and 2*ST*CS words follow: 8-byte aligned
+        full = reinterpret_cast<uint64_t*>(meta_k + ST * CS);
+        empty = full + ST;
+    }
+    // Every thread; false where a CTA of this launch already gave up.
+    __device__ __forceinline__ bool start(int consumers, const int* status) {
+        __shared__ int s_abort;
+        if (threadIdx.x == 0) {
+            s_abort = *(volatile const int*)status;
+            for (int b = 0; b < ST; ++b) {
+                mbar_init(&full[b], 1);
+                mbar_init(&empty[b], (unsigned)consumers);
+            }
+            asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        }
+        __syncthreads();
+        return s_abort == 0;
+    }
+};
+
+// The copy warp of a tile of TT samples from t0 and the trials of values
+// dv0 .. dv_last.
+template <int TT, int CS, int ST>
+__device__ __forceinline__ void tma_producer(const DedispArgs& a, const Pipe<CS, ST>& pipe, long long t0, float dv0,
+                                             float dv_last, int* status, int lane) {
+    const int nstages = (a.nchan + CS - 1) / CS;
+    float* slots = pipe.slots;
+    int* meta_off = pipe.meta_off;
+    float* meta_k = pipe.meta_k;
+    uint64_t *full = pipe.full, *empty = pipe.empty;
+    const int valid = (int)min((long long)TT, (long long)a.nout - t0);
+    int issued = 0;
+    bool ok = true;
+    const bool mine = lane < CS;
+    // the next stage's delay constants are on their way while this stage waits for its slot
+    float k_next = mine && lane < a.nchan ? a.dmshift[lane] : 0.0f;
+    const long long col0 = a.ring_len > 0 ? (a.t_base + t0) % a.ring_len : t0;
+    for (int st = 0; st < nstages && ok; ++st) {
+        const float k = k_next;
+        const int cn = (st + 1) * CS + lane;
+        if (mine && cn < a.nchan) k_next = a.dmshift[cn];
+        const int b = st % ST;
+        const unsigned round = (unsigned)(st / ST);
+        if (!mbar_wait_warp(&empty[b], (round & 1u) ^ 1u, a.wait_ns)) {
+            if (lane == 0) atomicExch(status, PV_ERR_TIMEOUT);
+            ok = false;
+            break;
+        }
+        if (a.stall && st == 0) {  // nothing completes this stage: its consumers' wait runs out
+            issued = st + 1;
+            continue;
+        }
+        const int c = st * CS + lane;
+        unsigned bytes = 0, piece1 = 0, piece2 = 0;
+        long long g_al = 0;
+        int tail = 0;  // linear rows: samples from piece1 on that are not copied in bulk
+        if (mine && c < a.nchan) {
+            const int s0 = pv_shift(k, dv0);
+            const int span = valid + pv_shift(k, dv_last) - s0;
+            int base;
+            if (a.ring_len > 0) {
+                const long long g0 = ring_column(col0 + s0, a.ring_len);
+                g_al = g0 & ~3LL;
+                base = (int)(g0 - g_al);
+                const unsigned n = (unsigned)((base + span + 3) & ~3);
+                piece1 = (unsigned)min((long long)n, a.ring_len - g_al);
+                piece2 = n - piece1;
+            } else {
+                // Positions in the whole buffer: aligned units up to the last readable sample
+                // (linear_end), the rest one by one, zeros beyond it.
+                const long long g0 = (long long)c * a.row_stride + t0 + s0;
+                g_al = g0 & ~3LL;
+                base = (int)(g0 - g_al);
+                const long long end = linear_end(a, c), want = (base + span + 3) & ~3;
+                const long long fit = end > g_al ? (end - g_al) & ~3LL : 0;
+                piece1 = (unsigned)min(want, fit);
+                tail = max(0, base + span - (int)piece1);
+            }
+            bytes = (piece1 + piece2) * 4u;
+            meta_off[b * CS + lane] = s0 - base;
+            meta_k[b * CS + lane] = k;
+            __threadfence_block();
+        }
+        for (unsigned m = __ballot_sync(0xffffffffu, tail > 0); m; m &= m - 1) {
+            const int l = __ffs(m) - 1;
+            const int first = __shfl_sync(0xffffffffu, (int)piece1, l), n = __shfl_sync(0xffffffffu, tail, l);
+            const long long g = __shfl_sync(0xffffffffu, g_al, l) + first;
+            const long long end = linear_end(a, st * CS + l);
+            float* dst = slots + (size_t)(b * CS + l) * a.slot + first;
+            for (int j = lane; j < n; j += 32) dst[j] = g + j < end ? a.in[g + j] : 0.0f;
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __threadfence_block();
+        }
+        unsigned total = bytes;
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+        __syncwarp();
+        if (lane == 0) mbar_arrive_expect_tx(&full[b], total);
+        __syncwarp();
+        if (bytes) {
+            const float* src = a.ring_len > 0 ? a.in + (long long)c * a.row_stride : a.in;
+            float* dst = slots + (size_t)(b * CS + lane) * a.slot;
+            if (piece1) bulk_g2s(dst, src + g_al, piece1 * 4u, &full[b]);
+            if (piece2) bulk_g2s(dst + piece1, src, piece2 * 4u, &full[b]);
+        }
+        issued = st + 1;
+    }
+    // Before the producer leaves, its last copies have landed (bounded):
+    // consumers that give up return at once, and the CTA's shared memory
+    // must not be released under copies in flight.
+    (void)ok;
+    for (int st = max(0, issued - ST); st < issued; ++st)
+        if (!(a.stall && st == 0))  // the withheld stage has no copies in flight
+            mbar_wait_warp(&full[st % ST], (unsigned)(st / ST) & 1u, pv::kDrainWaitNs);
+}
 
 template <int DMS, int R, int CS, int ST>
 __global__ void __launch_bounds__((DMS + 1) * 32)
 dedisperse_tma_kernel(const DedispArgs a, int* __restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int TT = 32 * R;
-    float* slots = reinterpret_cast<float*>(smem_raw);
-    int* meta_off = reinterpret_cast<int*>(slots + (size_t)ST * CS * a.slot);
-    float* meta_k = reinterpret_cast<float*>(meta_off + ST * CS);
-    // slot is a multiple of 4 floats and 2*ST*CS words follow: 8-byte aligned
-    uint64_t* full = reinterpret_cast<uint64_t*>(meta_k + ST * CS);
-    uint64_t* empty = full + ST;
+    Pipe<CS, ST> pipe(smem_raw, a.slot);
+    const float* slots = pipe.slots;
+    const int* meta_off = pipe.meta_off;
+    const float* meta_k = pipe.meta_k;
+    uint64_t *full = pipe.full, *empty = pipe.empty;
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long t0 = (long long)blockIdx.x * TT;
     const int d0 = blockIdx.y * DMS;
     const int d_last = min(d0 + DMS, a.tdms) - 1;
-    const float dv0 = pv_trial_value(d0, a.start, a.step);
-    const float dv_last = pv_trial_value(d_last, a.start, a.step);
     const int nstages = (a.nchan + CS - 1) / CS;
-
-    __shared__ int s_abort;
-    if (threadIdx.x == 0) {
-        // a launch in which some CTA already gave up stops here
-        s_abort = *(volatile int*)status;
-        for (int b = 0; b < ST; ++b) {
-            mbar_init(&full[b], 1);
-            mbar_init(&empty[b], DMS);
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    }
-    __syncthreads();
-    if (s_abort != 0) return;
-
+    if (!pipe.start(DMS, status)) return;
     if (warp == DMS) {
-        // ---------------- producer ----------------
-        const int valid = (int)min((long long)TT, (long long)a.nout - t0);
-        int issued = 0;
-        bool ok = true;
-        const bool mine = lane < CS;
-        // the next stage's delay constants are on their way while this stage waits for its slot
-        float k_next = mine && lane < a.nchan ? a.dmshift[lane] : 0.0f;
-        const long long col0 = a.ring_len > 0 ? (a.t_base + t0) % a.ring_len : t0;
-        for (int st = 0; st < nstages && ok; ++st) {
-            const float k = k_next;
-            const int cn = (st + 1) * CS + lane;
-            if (mine && cn < a.nchan) k_next = a.dmshift[cn];
-            const int b = st % ST;
-            const unsigned round = (unsigned)(st / ST);
-            if (!mbar_wait_warp(&empty[b], (round & 1u) ^ 1u, a.wait_ns)) {
-                if (lane == 0) atomicExch(status, PV_ERR_TIMEOUT);
-                ok = false;
-                break;
-            }
-            if (a.stall && st == 0) {  // nothing completes this stage: its consumers' wait runs out
-                issued = st + 1;
-                continue;
-            }
-            const int c = st * CS + lane;
-            unsigned bytes = 0, piece1 = 0, piece2 = 0;
-            long long g_al = 0;
-            int tail = 0;  // linear rows: samples from piece1 on that are not copied in bulk
-            if (mine && c < a.nchan) {
-                const int s0 = pv_shift(k, dv0);
-                const int span = valid + pv_shift(k, dv_last) - s0;
-                int base;
-                if (a.ring_len > 0) {
-                    const long long g0 = ring_column(col0 + s0, a.ring_len);
-                    g_al = g0 & ~3LL;
-                    base = (int)(g0 - g_al);
-                    const unsigned n = (unsigned)((base + span + 3) & ~3);
-                    piece1 = (unsigned)min((long long)n, a.ring_len - g_al);
-                    piece2 = n - piece1;
-                } else {
-                    // Positions in the whole buffer: aligned units up to the last readable sample
-                    // (linear_end), the rest one by one, zeros beyond it.
-                    const long long g0 = (long long)c * a.row_stride + t0 + s0;
-                    g_al = g0 & ~3LL;
-                    base = (int)(g0 - g_al);
-                    const long long end = linear_end(a, c), want = (base + span + 3) & ~3;
-                    const long long fit = end > g_al ? (end - g_al) & ~3LL : 0;
-                    piece1 = (unsigned)min(want, fit);
-                    tail = max(0, base + span - (int)piece1);
-                }
-                bytes = (piece1 + piece2) * 4u;
-                meta_off[b * CS + lane] = s0 - base;
-                meta_k[b * CS + lane] = k;
-                __threadfence_block();
-            }
-            for (unsigned m = __ballot_sync(0xffffffffu, tail > 0); m; m &= m - 1) {
-                const int l = __ffs(m) - 1;
-                const int first = __shfl_sync(0xffffffffu, (int)piece1, l), n = __shfl_sync(0xffffffffu, tail, l);
-                const long long g = __shfl_sync(0xffffffffu, g_al, l) + first;
-                const long long end = linear_end(a, st * CS + l);
-                float* dst = slots + (size_t)(b * CS + l) * a.slot + first;
-                for (int j = lane; j < n; j += 32) dst[j] = g + j < end ? a.in[g + j] : 0.0f;
-                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-                __threadfence_block();
-            }
-            unsigned total = bytes;
-#pragma unroll
-            for (int o = 16; o >= 1; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-            __syncwarp();
-            if (lane == 0) mbar_arrive_expect_tx(&full[b], total);
-            __syncwarp();
-            if (bytes) {
-                const float* src = a.ring_len > 0 ? a.in + (long long)c * a.row_stride : a.in;
-                float* dst = slots + (size_t)(b * CS + lane) * a.slot;
-                if (piece1) bulk_g2s(dst, src + g_al, piece1 * 4u, &full[b]);
-                if (piece2) bulk_g2s(dst + piece1, src, piece2 * 4u, &full[b]);
-            }
-            issued = st + 1;
-        }
-        // Before the producer leaves, its last copies have landed (bounded):
-        // consumers that give up return at once, and the CTA's shared memory
-        // must not be released under copies in flight.
-        (void)ok;
-        for (int st = max(0, issued - ST); st < issued; ++st)
-            if (!(a.stall && st == 0))  // the withheld stage has no copies in flight
-                mbar_wait_warp(&full[st % ST], (unsigned)(st / ST) & 1u, pv::kDrainWaitNs);
+        tma_producer<TT, CS, ST>(a, pipe, t0, pv_trial_value(d0, a.start, a.step),
+                                 pv_trial_value(d_last, a.start, a.step), status, lane);
         return;
     }
 
@@ -901,6 +930,83 @@ __device__ __forceinline__ void pair_dispatch(const float* __restrict__ row, int
 #undef PV_PAIR
 }
 
+// One beam's rows by trial pairs: tiles of 2 * PAIRS trials and 1056 samples,
+// one pair per warp, copied as for dedisperse_tma_kernel.  Where a pair's
+// delays differ by few samples most words serve both trials (0.5 words per
+// add at equal delays, 0.58 at a difference of 5), which lifts the bound of
+// one shared-memory word per add; 126 registers a thread leave 16 warps an SM,
+// 7 + 1 in each of two CTAs or 4 + 1 in each of three.  One CTA of 14 pair
+// warps (7 x 2112 samples) was as fast on full grids and slower on all others;
+// 6 warps in two CTAs or 12 in one spill.  Measured: 1024 trials x 1024
+// channels x 8192 samples 979 -> 833 us, the tile rule below has more.
+template <int PAIRS, int CS, int ST>
+__global__ void __launch_bounds__((PAIRS + 1) * 32, 16 / (PAIRS + 1))
+dedisperse_tma_pair_kernel(const DedispArgs a, int* __restrict__ status) {
+    constexpr int TT = 32 * kPairS;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    Pipe<CS, ST> pipe(smem_raw, a.slot);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long t0 = (long long)blockIdx.x * TT;
+    const int d0 = blockIdx.y * 2 * PAIRS;
+    const int d_last = min(d0 + 2 * PAIRS, a.tdms) - 1;
+    const int nstages = (a.nchan + CS - 1) / CS;
+    if (!pipe.start(PAIRS, status)) return;
+    if (warp == PAIRS) {
+        tma_producer<TT, CS, ST>(a, pipe, t0, pv_trial_value(d0, a.start, a.step),
+                                 pv_trial_value(d_last, a.start, a.step), status, lane);
+        return;
+    }
+    const int da = d0 + 2 * warp;
+    const bool act_a = da <= d_last, act_b = da + 1 <= d_last;
+    const int lane_t = kPairS * lane;  // the lane's first sample in the tile
+    const float dva = pv_trial_value(min(da, d_last), a.start, a.step);
+    const float dvb = pv_trial_value(min(da + 1, d_last), a.start, a.step);
+    float a0[kPairS], a1[kPairS];
+#pragma unroll
+    for (int j = 0; j < kPairS; ++j) a0[j] = a1[j] = 0.0f;
+    for (int st = 0; st < nstages; ++st) {
+        const int b = st % ST;
+        if (!mbar_wait_warp(&pipe.full[b], (unsigned)(st / ST) & 1u, a.wait_ns)) {
+            if (lane == 0) atomicExch(status, PV_ERR_TIMEOUT);
+            return;
+        }
+        if (act_a) {
+            const int c_end = min(CS, a.nchan - st * CS);
+            int my_oa = 0, my_dl = 0;
+            if (lane < c_end) {
+                const float k = pipe.meta_k[b * CS + lane];
+                const int mo = pipe.meta_off[b * CS + lane];
+                my_oa = min(pv_shift(k, dva) - mo, a.slot - TT);
+                my_dl = min(pv_shift(k, dvb) - mo, a.slot - TT) - my_oa;
+            }
+            int oa = __shfl_sync(0xffffffffu, my_oa, 0);
+            int dl = __shfl_sync(0xffffffffu, my_dl, 0);
+            for (int j = 0; j < c_end; ++j) {
+                const int oa_n = __shfl_sync(0xffffffffu, my_oa, (j + 1) & 31);
+                const int dl_n = __shfl_sync(0xffffffffu, my_dl, (j + 1) & 31);
+                const float* row = pipe.slots + (size_t)(b * CS + j) * a.slot + oa + lane_t;
+                float w[kPairS];
+#pragma unroll
+                for (int q = 0; q < kPairS; ++q) w[q] = row[q];
+                pair_dispatch<15>(row, dl, w, a0, a1);
+                oa = oa_n;
+                dl = dl_n;
+            }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&pipe.empty[b]);
+    }
+    float* o = a.out + (long long)da * a.out_stride;
+#pragma unroll
+    for (int j = 0; j < kPairS; ++j) {
+        const long long t = t0 + lane_t + j;
+        if (t < a.nout) {
+            if (act_a) o[t] = a0[j];
+            if (act_b) o[a.out_stride + t] = a1[j];
+        }
+    }
+}
+
 // PAIRS trial pairs per tile (2 * PAIRS trials) and HALVES parts of the
 // time tile (HALVES x 1056 samples): consumer warp w takes pair w % PAIRS in
 // part w / PAIRS.  8 x 1: 8 consumer warps; 6 x 2: 12; 7 x 2: 14, more warps
@@ -1069,6 +1175,20 @@ int launch_dedisperse_tma(DedispArgs a, int spread, int* status, cudaStream_t s)
     return pv::check_launch("dedisperse_tma_kernel");
 }
 
+template <int PAIRS, int CS, int ST>
+int launch_dedisperse_pair(DedispArgs a, int spread, int* status, cudaStream_t s) {
+    constexpr int TT = 32 * kPairS;
+    a.slot = (TT + spread + 8 + 3) & ~3;
+    const size_t smem = (size_t)ST * CS * a.slot * sizeof(float) + (size_t)ST * CS * 8 + 8 +
+                        (size_t)2 * ST * sizeof(uint64_t);
+    auto kern = dedisperse_tma_pair_kernel<PAIRS, CS, ST>;
+    PV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+            "cudaFuncSetAttribute(dedisperse_tma_pair)");
+    dim3 grid((unsigned)pv::ceil_div<long long>(a.nout, TT), (unsigned)pv::ceil_div(a.tdms, 2 * PAIRS));
+    kern<<<grid, (PAIRS + 1) * 32, smem, s>>>(a, status);
+    return pv::check_launch("dedisperse_tma_pair_kernel");
+}
+
 }  // namespace
 
 namespace pv {
@@ -1078,10 +1198,13 @@ static size_t tma_smem(int st, int cs, int slot_floats) {
     return (size_t)st * cs * slot_floats * sizeof(float) + (size_t)st * cs * 8 + 8 + 2 * st * 8;
 }
 
-// Tiles of the pipelined kernel: trials x samples, channels per stage, stages.
+// Tiles of the pipelined kernels: trials x samples, channels per stage,
+// stages; for trial pairs how many CTAs the registers let an SM hold.
 struct TmaTile {
     int dms, tt, cs, st;
-    float rate;  // adds per second with every SM busy, of the first one's
+    float rate;   // adds per second with every SM busy, of the first one's
+    float slope;  // of pairs: what the rate loses per sample of a pair's mean delay difference
+    int resident;
 };
 // Tadd/s on 512 trials x 3904 channels x 16384 samples (110-158 MHz, DM 125:
 // tile spreads of 16 trials up to 1050 samples) / 512 x 512 x 10976 / 300 x
@@ -1093,27 +1216,68 @@ struct TmaTile {
 // Wide tiles need the fewest copied samples per add, narrow ones fill the SMs
 // where the wide ones are few; 16 x 4 in 2-channel stages holds spreads that
 // 8-channel stages do not.
-constexpr TmaTile kTmaTiles[] = {{16, 1024, 8, 2, 1.0f}, {16, 1024, 2, 4, 0.93f}, {8, 1024, 8, 2, 0.95f},
-                                 {8, 256, 16, 2, 0.93f}};
+// Trial pairs read fewer words per add, the fewer the smaller the pair's delay
+// difference, but only 12 or 14 warps of 66 sums fit an SM.  us of the best
+// one-trial tile / 14 x 1056 / 8 x 1056, by the mean difference:
+//   1024 trials x 4096 channels x 16384, 0.0   7504  6087  6220
+//   1024 x 512 x 16000, 2.6                     968   897   856
+//   1024 x 1024 x 8192, 3.3                     979   833   933
+//   1024 x 976 x 32000, 4.5                    3491  3051  3025
+//    512 x 512 x 10976, 5.2                     360   368   344
+//   1024 x 1024 x 8192, 13.3                   1010   956  1252
+//    200 x 768 x 12000, 23.6                    224   398   275
+constexpr TmaTile kTmaTiles[] = {{16, 1024, 8, 2, 1.0f, 0.0f, 0},  {16, 1024, 2, 4, 0.93f, 0.0f, 0},
+                                 {8, 1024, 8, 2, 0.95f, 0.0f, 0},  {8, 256, 16, 2, 0.93f, 0.0f, 0},
+                                 {14, 1056, 8, 2, 1.27f, 0.02f, 2}, {8, 1056, 8, 2, 1.28f, 0.03f, 3}};
+constexpr int kOneTrialTiles = 4, kTiles = 6;
 
 // The tile with the least expected time, -1 if none fits: the busiest SM's
 // share of the adds, at a rate that falls where a tile copies more than 0.55
-// bytes per add through L2.
+// bytes per add through L2.  Delays differ most in the lowest channel: half
+// that difference, a seventh of the spread of eight trials, stands for a
+// pair's mean one (measured: 0.4 to 0.5 of it).  A last round that does not
+// fill the SM's residency runs at the 0.6th power of the part it fills
+// (measured for 1 of 2 and 2 of 3 CTAs: 0.65 and 0.74).
 template <typename F>
 int tma_tile(int tdms, int nout, long long ring_len, F spread) {
+    const auto smem_of = [](const TmaTile& t, int sp) { return tma_smem(t.st, t.cs, (t.tt + sp + 8 + 3) & ~3); };
+    // two stages fit, and every copy (span + 16-byte rounding) in one ring turn
+    const auto fits = [&](const TmaTile& t, int sp) {
+        return smem_of(t, sp) <= 220 * 1024 &&
+               (ring_len <= 0 || ring_len >= (long long)std::min(t.tt, nout) + sp + 8);
+    };
+    const auto time_of = [&](const TmaTile& t, int sp, double rate, double busiest) {
+        const double copied = 4.0 * (t.tt + sp) / ((double)t.tt * t.dms);
+        return busiest * t.dms * t.tt / rate * std::max(1.0, copied / 0.55);
+    };
+    const auto busiest_of = [&](const TmaTile& t) {
+        return std::ceil((double)ceil_div(tdms, t.dms) * ceil_div(nout, t.tt) / sm_count());
+    };
     int best = -1;
     double best_t = 0.0;
-    for (int v = 0; v < 4; ++v) {
+    for (int v = 0; v < kOneTrialTiles; ++v) {
         const TmaTile& t = kTmaTiles[v];
         const int sp = spread(t.dms);
-        if (tma_smem(t.st, t.cs, (t.tt + sp + 8 + 3) & ~3) > 220 * 1024) continue;
-        // every copy (span + 16-byte rounding) must fit in one ring turn
-        if (ring_len > 0 && ring_len < (long long)std::min(t.tt, nout) + sp + 8) continue;
-        const double tiles = (double)ceil_div(tdms, t.dms) * ceil_div(nout, t.tt);
-        const double busiest = std::ceil(tiles / sm_count());
-        const double copied = 4.0 * (t.tt + sp) / ((double)t.tt * t.dms);
-        const double time = busiest * t.dms * t.tt / t.rate * std::max(1.0, copied / 0.55);
+        if (!fits(t, sp)) continue;
+        const double time = time_of(t, sp, t.rate, busiest_of(t));
         if (best < 0 || time < best_t) {
+            best = v;
+            best_t = time;
+        }
+    }
+    const double diff = spread(8) / 7.0;
+    for (int v = kOneTrialTiles; v < kTiles && best >= 0; ++v) {
+        const TmaTile& t = kTmaTiles[v];
+        const double rate = t.rate - t.slope * 0.5 * diff;
+        const int sp = (int)(diff * (t.dms - 1));  // exact only where it could win: the host pays for each spread
+        if (rate <= 0.5) continue;
+        const double held = std::min(t.resident, (int)(227 * 1024 / (smem_of(t, sp) + 1024)));
+        if (held < 1.0) continue;
+        double busiest = busiest_of(t);
+        const double part = std::fmod(busiest, held) / held;
+        if (part > 0.0) busiest += held * (std::pow(part, 0.4) - part);
+        const double time = time_of(t, sp, rate * std::pow(held / t.resident, 0.6), busiest);
+        if (time < best_t && fits(t, spread(t.dms))) {
             best = v;
             best_t = time;
         }
@@ -1146,7 +1310,9 @@ int dedisperse_device(float* out, long long out_stride, const float* in, long lo
             if (v == 0) return launch_dedisperse_tma<16, 32, 8, 2>(a, sp, status, s);
             if (v == 1) return launch_dedisperse_tma<16, 32, 2, 4>(a, sp, status, s);
             if (v == 2) return launch_dedisperse_tma<8, 32, 8, 2>(a, sp, status, s);
-            return launch_dedisperse_tma<8, 8, 16, 2>(a, sp, status, s);
+            if (v == 3) return launch_dedisperse_tma<8, 8, 16, 2>(a, sp, status, s);
+            if (v == 4) return launch_dedisperse_pair<7, 8, 2>(a, sp, status, s);
+            return launch_dedisperse_pair<4, 8, 2>(a, sp, status, s);
         }
     }
     const int spread16 = spread(16);
@@ -1660,10 +1826,14 @@ extern "C" int pv_dedisperse_ex(float* d_out, long long out_stride, const float*
             return PV_ERR_ARG;
         }
     }
-    return pv::dedisperse_device(
-        d_out, out_stride, d_in, row_stride, row_len, 0, 0, nchans, nout, tdms, d_dmshift,
-        [&](int dms) { return delay_spread(h, tdms, dms, start_over_tsamp, step_over_tsamp); }, start_over_tsamp,
-        step_over_tsamp, s, status);
+    std::map<int, int> spreads;  // each is asked for several times
+    const auto spread = [&](int dms) {
+        const auto it = spreads.find(dms);
+        if (it != spreads.end()) return it->second;
+        return spreads[dms] = delay_spread(h, tdms, dms, start_over_tsamp, step_over_tsamp);
+    };
+    return pv::dedisperse_device(d_out, out_stride, d_in, row_stride, row_len, 0, 0, nchans, nout, tdms, d_dmshift,
+                                 spread, start_over_tsamp, step_over_tsamp, s, status);
 }
 
 extern "C" int pv_dedisperse(float* d_out, long long out_bytes, const float* d_in,

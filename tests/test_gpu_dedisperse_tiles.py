@@ -88,3 +88,34 @@ def test_ring_rows(pv, oracle, cuda, case):
         got = plan.run(torch.from_numpy(np.ascontiguousarray(x)).to(cuda), nout, ring_len=ring, t_base=base)
         assert np.array_equal(got.cpu().numpy(), want)
     assert plan.status() == 0
+
+
+PAIR_CASES = [
+    # Trial pairs, delay differences of 0 to 28 samples (from 16 on each
+    # trial reads its own words): rows enough to fill every SM.  14 x 1056
+    # on a grid of one and of two trials more than its tiles, 8 x 1056 on an odd one; a last
+    # sample tile of one sample and one that is full.
+    (9, 1024, 8449, 150.0, -0.05, 30.0),
+    (17, 1023, 8448, 150.0, -0.05, 5000.0),
+    (17, 1024, 8448, 150.0, -0.05, 14000.0),
+    (20, 513, 10976, 150.0, -0.05, 4600.0),
+    (3, 4097, 9000, 1300.0, -0.04, 0.0),
+]
+
+
+@pytest.mark.parametrize("ring", [False, True])
+@pytest.mark.parametrize("case", PAIR_CASES)
+def test_trial_pairs(pv, oracle, cuda, case, ring):
+    import torch
+    nchan, tdms, nout = case[:3]
+    k, start, step, ms, rng = _case(pv, oracle, case, 3)
+    width = nout + ms + (1100 if ring else 1)
+    width = (width + 3) // 4 * 4 if ring else width
+    x = rng.standard_normal((nchan, width)).astype(np.float32)
+    want = oracle.dedisperse(x, nout, tdms, k, start, step)
+    plan = pv.DedispPlan(k, tdms, float(start), float(step))
+    base = width - 7 if ring else 0
+    xd = torch.from_numpy(np.ascontiguousarray(np.roll(x, base, axis=1))).to(cuda)
+    got = plan.run(xd, nout, ring_len=width if ring else 0, t_base=base)
+    assert np.array_equal(got.cpu().numpy(), want)
+    assert plan.status() == 0

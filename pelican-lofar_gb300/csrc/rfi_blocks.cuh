@@ -27,11 +27,12 @@
 // The margin moves over a block, and a channel whose value lies between the
 // expected and the exact margin fails the proof: rare in quiet data, common
 // with strong RFI whose values reach down to the margin while the averages
-// drift.  After a few failures the scan stops at the spectrum it has reached
-// and writes down the margins that the recorded sums predict for the rest; a
-// second rfi_stats_kernel clips the unproven spectra with those, and a second
-// rfi_scan_kernel goes on from there.  Both return at once where the first
-// scan was enough.
+// drift.  At the first failure the scan works out, in FP32, the margins that
+// the recorded sums predict for the rest of the block.  Where they would fail
+// more records it writes them down and leaves the rest to a second
+// rfi_stats_kernel, which clips the unproven spectra with them, and a second
+// rfi_scan_kernel; so does a scan that meets more failures than predicted.
+// Both return at once where the first scan was enough.
 //
 // The running averages x <- fl(fl(x - a) + b) are rounded at every step, and
 // every bit of them is kept: while x stays in one binade, x is an integer
@@ -81,9 +82,12 @@ constexpr int kZeroList = 2048;
 // value; after the first scan, the spectrum it reached, whether the second
 // pass is wanted and whether a spectrum of the block has filled channels.
 constexpr int kHdrNum = 0, kHdrZeros = 1, kHdrPos = 2, kHdrRedo = 3, kHdrFilled = 4, kHdrWords = 8;
-// Failed proofs that the first scan does over by itself (6 us each); beyond
-// that a second pass over the unproven spectra (about 20 us) costs less.
-constexpr int kAloneMax = 4;
+// Failed proofs that the first scan does over by itself.  Each costs a scan of
+// one spectrum and a group begun again, a second pass 3 to 15 us of statistics:
+// the forecast at the first failure tells (more failures than kForecastMax,
+// itself included, want the pass), and where it was wrong kAloneMax does.
+constexpr int kForecastMax = 2, kAloneMax = 4;
+constexpr int kForecast = 4;  // spectra per thread of a forecast: a whole block at once
 constexpr int kSerial = 256;  // spectra of a group whose averages are added one by one, at most
 
 // Order-preserving map of a float's bits to int (NaN excluded by the callers).
@@ -737,7 +741,7 @@ __device__ __forceinline__ int scan_group(ScanShared& sh, const RfiConfig& cfg, 
         double a = 0.0, b = 0.0, Mp;
         if (act) {
             a = bufs.mean_buf[wrap_h(mhead + k, H)] * inv_h;
-            if (k > 0 || (predict && i > 0)) b = entry(w.rec[i + k - 1]);
+            if (k > 0) b = widen(w.rec[i + k - 1].ssum);
             else b = bufs.mean_buf[wrap_h(mhead + H - 1, H)];
             b = b * inv_h;
         }
@@ -748,7 +752,7 @@ __device__ __forceinline__ int scan_group(ScanShared& sh, const RfiConfig& cfg, 
         if (act) {
             a = bufs.rms_buf[wrap_h(rhead + k, H)] * inv_h;
             if (k > 0) b = sh.E[k - 1];
-            else b = predict ? E : bufs.rms_buf[wrap_h(rhead + H - 1, H)];
+            else b = bufs.rms_buf[wrap_h(rhead + H - 1, H)];
             b = b * inv_h;
         }
         bad |= !slide(sh, st.rms_run, a, b, k, m, mode, 1, R, Mp);
@@ -912,25 +916,119 @@ __device__ __forceinline__ int scan_group(ScanShared& sh, const RfiConfig& cfg, 
     return f;
 }
 
-// The expected margins of spectra i..n-1 from the records, for the second
-// statistics pass.  The shared state moves on approximately.
-__device__ __forceinline__ void scan_predict(ScanShared& sh, const RfiConfig& cfg, const RfiBuffers& bufs,
-                                             const RfiWork& w, const float* rows, long long spec_elems,
-                                             const Geo& geo, int i, int n) {
-    const int H = cfg.history;
-    while (i < n) {
-        __syncthreads();
-        const int rs = sh.st.rms_size;
-        int m = min(min(kScanThreads, n - i), H);
-        if (rs < H) m = min(m, max(H - 1 - rs, 1));
-        bool c, u;
-        scan_group(sh, cfg, bufs, w, rows, spec_elems, geo, i, m, false, kPredict, c, u);
-        i += m;
-        if (rs < H && sh.st.rms_size >= H - 1 && threadIdx.x == 0) {  // the histories are full
-            sh.st.rms_size = sh.st.mean_size = H;
-            sh.st.inv_mor = sh.st.rms_run / sh.st.mean_run;
+// FP32 prefix sums over kForecast * kScanThreads values, v[j] being number
+// j * kScanThreads + thread: what lies before each (before) and up to it (v).
+// wt: a word per warp and j, not in use since the last barrier.
+__device__ __forceinline__ void block_scan_f(float (&v)[kForecast], float (&before)[kForecast], float* wt) {
+    constexpr int NW = kScanThreads / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float x[kForecast];
+#pragma unroll
+    for (int j = 0; j < kForecast; ++j) x[j] = v[j];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+        for (int j = 0; j < kForecast; ++j) {
+            const float y = __shfl_up_sync(0xffffffffu, x[j], o);
+            if (lane >= o) x[j] += y;
         }
+    if (lane == 31)
+#pragma unroll
+        for (int j = 0; j < kForecast; ++j) wt[j * NW + warp] = x[j];
+    __syncthreads();
+    static_assert(kForecast * NW == 64, "two warp totals a lane");
+    const float t0 = wt[2 * lane], t1 = wt[2 * lane + 1];
+    float t = t0 + t1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float y = __shfl_up_sync(0xffffffffu, t, o);
+        if (lane >= o) t += y;
     }
+    // t: the totals up to number 2 * lane + 1
+#pragma unroll
+    for (int j = 0; j < kForecast; ++j) {
+        const int q = j * NW + warp;
+        const float upto = __shfl_sync(0xffffffffu, t, q >> 1), odd = __shfl_sync(0xffffffffu, t1, q >> 1);
+        const float own = __shfl_sync(0xffffffffu, t0, q >> 1);
+        const float base = (q & 1) ? upto - odd : upto - odd - own;
+        before[j] = base + (x[j] - v[j]);
+        v[j] = base + x[j];
+    }
+}
+
+// The expected margins of spectra i..n-1 with full histories, from the records
+// and in FP32, written to RfiWork::out; returns how many records they do not
+// prove.  exact: the shared state is the one before spectrum i (else the
+// newest history entry is the record's before it).  The state and the
+// histories stay as they are.  18k cycles for 2048 spectra; by the exact
+// scan's groups, as the adaptive phase still does it, 48k.
+__device__ __forceinline__ int scan_forecast(ScanShared& sh, const RfiConfig& cfg, const RfiBuffers& bufs,
+                                             const RfiWork& w, int i, int n, bool exact) {
+    const int tid = threadIdx.x;
+    const int H = cfg.history;
+    const RfiState& st = sh.st;
+    const bool flat = cfg.deg == 0 && bufs.killed == nullptr;
+    const float inv_h = narrow(cfg.inv_h), inv_mor = narrow(st.inv_mor), mean_first = narrow(st.mean_run);
+    const float inv_scale = 1.0f / cfg.scale;
+    // a rejected spectrum leaves the mean where it is
+    const float loud = mean_first + 1.01f * cfg.sr * st.bp_rms * narrow(cfg.inv_sqrt_nbins);
+    float mean0 = mean_first, rms0 = narrow(st.rms_run);
+    int mhead = st.mean_head, rhead = st.rms_head;
+    __syncthreads();
+    if (tid == 0) sh.first_bad = 0;
+    while (i < n) {
+        const int m = min(min(kForecast * kScanThreads, n - i), H);
+        float dm[kForecast], dr[kForecast], mb[kForecast], rb[kForecast], old[kForecast];
+#pragma unroll
+        for (int j = 0; j < kForecast; ++j) {
+            const int k = j * kScanThreads + tid;
+            dm[j] = old[j] = 0.0f;
+            if (k < m) {
+                float b;
+                if (k > 0 || !exact) {
+                    const SpecRec& q = w.rec[i + k - 1];
+                    b = H >= 1000 && (q.ssum > loud || q.bad_bands >= 4) ? mean_first : q.ssum;
+                } else {
+                    b = narrow(bufs.mean_buf[wrap_h(mhead + H - 1, H)]);
+                }
+                dm[j] = (b - narrow(bufs.mean_buf[wrap_h(mhead + k, H)])) * inv_h;
+                old[j] = narrow(bufs.rms_buf[wrap_h(rhead + k, H)]);
+            }
+        }
+        block_scan_f(dm, mb, sh.rf);
+#pragma unroll
+        for (int j = 0; j < kForecast; ++j) {
+            // the entry |mean / meanOverRMS| of the spectrum before, to one step of the mean
+            const float b = fabsf((mean0 + mb[j]) * inv_mor);
+            dr[j] = j * kScanThreads + tid < m ? (b - old[j]) * inv_h : 0.0f;
+        }
+        block_scan_f(dr, rb, sh.mf);
+        int bad = 0;
+#pragma unroll
+        for (int j = 0; j < kForecast; ++j) {
+            const int k = j * kScanThreads + tid;
+            if (k >= m) continue;
+            const float mean = mean0 + dm[j], rms = rms0 + dr[j], margin = cfg.cr * rms;
+            const float p = st.params0 + (mean0 + mb[j] - st.bp_mean) * inv_scale;
+            bad += rfi_proven(cfg, flat, w.rec[i + k], 0.0f, margin, p) ? 0 : 1;
+            w.out[i + k] = SpecOut{0.0f, margin, p, mean, 0, {0, 0, 0}};
+            if (k == m - 1) {
+                sh.pi[0] = mean;
+                sh.pi[1] = rms;
+            }
+        }
+        bad = __reduce_add_sync(0xffffffffu, bad);
+        if ((tid & 31) == 0 && bad) atomicAdd(&sh.first_bad, bad);
+        __syncthreads();
+        mean0 = sh.pi[0];
+        rms0 = sh.pi[1];
+        i += m;
+        mhead = wrap_h(mhead + m, H);
+        rhead = wrap_h(rhead + m, H);
+        exact = false;
+        __syncthreads();
+    }
+    return sh.first_bad;
 }
 
 template <int P>
@@ -963,61 +1061,87 @@ __device__ __forceinline__ void rfi_scan_body(const RfiConfig& cfg, const RfiBuf
     int serial = 0, grow = 32;     // spectra of the next group if its averages are added one by one
     int failed = 0;
     bool redo = false;
-    while (i < n) {
+    for (;;) {
+        bool ask = false;
+        while (i < n) {
+            __syncthreads();
+            const int rs = sh.st.rms_size, num = sh.st.num;
+            // A group ends before the statistics' reset and before the histories are full; in the steady phase
+            // its oldest entries are older than the group.
+            int m = min(kScanThreads, n - i);
+            if (num == 0) m = 0;
+            else m = min(m, 10 * H - num);
+            if (rs < H) m = flat ? min(m, H - 1 - rs) : 0;
+            else m = min(m, H);
+            // averages that are 0, not finite or tiny have no usable binade
+            const RfiState& st = sh.st;
+            if (!binade64(rs < H ? st.rms_acc : st.rms_run).ok || !binade64(rs < H ? st.mean_acc : st.mean_run).ok) m = 0;
+            if (alone > 0) {
+                --alone;
+                m = 0;
+            }
+            if (m > 0) {
+                if (serial) m = min(m, serial);
+                bool chain, unproven;
+                const int f = scan_group(sh, cfg, bufs, w, rows, spec_elems, geo, i, m, filled,
+                                         serial ? kOneByOne : kParallel, chain, unproven);
+                i += f;
+                if (chain) {  // past a half-way case; longer where they come again at once (x near a binade's end)
+                    grow = f < 64 ? min(2 * grow, kSerial) : 32;
+                    serial = grow;
+                    continue;
+                }
+                serial = 0;
+                if (f == m) {
+                    streak = 0;
+                    continue;
+                }
+                if (unproven && !second && n - i > kAloneMax) {
+                    ++failed;
+                    if ((failed == 1 && rs >= H) || failed > kAloneMax) {
+                        ask = true;
+                        break;
+                    }
+                }
+                // groups that prove nothing are tried less and less often
+                streak = f == 0 ? min(streak + 1, 6) : 0;
+                alone = f == 0 ? (1 << streak) - 1 : 0;
+            }
+            scan_one<P>(sh, cfg, bufs, w, rows + (long long)i * spec_elems, geo, i);
+            filled |= sh.fill != 0 && sh.filled != 0;
+            ++i;
+        }
+        if (!ask) break;
+        redo = failed > kAloneMax;
         __syncthreads();
-        const int rs = sh.st.rms_size, num = sh.st.num;
-        // A group ends before the statistics' reset and before the histories are full; in the steady phase
-        // its oldest entries are older than the group.
-        int m = min(kScanThreads, n - i);
-        if (num == 0) m = 0;
-        else m = min(m, 10 * H - num);
-        if (rs < H) m = flat ? min(m, H - 1 - rs) : 0;
-        else m = min(m, H);
-        // averages that are 0, not finite or tiny have no usable binade
-        const RfiState& st = sh.st;
-        if (!binade64(rs < H ? st.rms_acc : st.rms_run).ok || !binade64(rs < H ? st.mean_acc : st.mean_run).ok) m = 0;
-        if (alone > 0) {
-            --alone;
-            m = 0;
+        if (tid == 0) *bufs.state = sh.st;  // before spectrum i; with a second pass the shared one moves on
+        int at = i;
+        while (at < n && sh.st.rms_size < H) {  // a second pass: approximately through the adaptive phase
+            __syncthreads();
+            const int rs = sh.st.rms_size;
+            const int m = min(min(kScanThreads, n - at), max(H - 1 - rs, 1));
+            bool c, u;
+            scan_group(sh, cfg, bufs, w, rows, spec_elems, geo, at, m, false, kPredict, c, u);
+            at += m;
+            if (sh.st.rms_size >= H - 1 && tid == 0) {  // the histories are full
+                sh.st.rms_size = sh.st.mean_size = H;
+                sh.st.inv_mor = sh.st.rms_run / sh.st.mean_run;
+            }
+            __syncthreads();
         }
-        if (m > 0) {
-            if (serial) m = min(m, serial);
-            bool chain, unproven;
-            const int f = scan_group(sh, cfg, bufs, w, rows, spec_elems, geo, i, m, filled,
-                                     serial ? kOneByOne : kParallel, chain, unproven);
-            i += f;
-            if (chain) {  // past a half-way case; longer where they come again at once (x near a binade's end)
-                grow = f < 64 ? min(2 * grow, kSerial) : 32;
-                serial = grow;
-                continue;
-            }
-            serial = 0;
-            if (f == m) {
-                streak = 0;
-                continue;
-            }
-            if (unproven && !second && ++failed > kAloneMax && n - i > kAloneMax) {
-                redo = true;
-                break;
-            }
-            // groups that prove nothing are tried less and less often
-            streak = f == 0 ? min(streak + 1, 6) : 0;
-            alone = f == 0 ? (1 << streak) - 1 : 0;
-        }
-        scan_one<P>(sh, cfg, bufs, w, rows + (long long)i * spec_elems, geo, i);
-        filled |= sh.fill != 0 && sh.filled != 0;
-        ++i;
+        if (at < n && scan_forecast(sh, cfg, bufs, w, at, n, at == i) > kForecastMax) redo = true;
+        if (redo) break;
+        alone = 1;
     }
     __syncthreads();
     if (tid == 0) {
-        *bufs.state = sh.st;
+        if (!redo) *bufs.state = sh.st;
         if (!second) {
             w.hdr[kHdrPos] = i;
             w.hdr[kHdrRedo] = redo ? 1 : 0;
             w.hdr[kHdrFilled] = filled ? 1 : 0;
         }
     }
-    if (redo) scan_predict(sh, cfg, bufs, w, rows, spec_elems, geo, i, n);
 }
 
 // ---------------------------------------------------------------------------

@@ -132,3 +132,20 @@ def test_rejected_until_the_reset(pv, oracle, cuda):
     data[1005:] *= 3.0
     bp = make_bp_text(nsub * nchan, START, WIDTH, 1000.0, 50.0)
     _run(pv, oracle, cuda, data, (9000,), bp, 1000, sr=0.5)
+
+
+@pytest.mark.parametrize("hits,history", [(2, 2500), (30, 2500), (3000, 2500), (30, 1100)])
+def test_few_and_many_failures_with_full_histories(pv, oracle, cuda, hits, history):
+    """Spectra with a fifth of their channels scattered around the margin: a
+    block with one or two failed proofs goes on by itself, one with many is
+    forecast from the first of them on, in one go or (a history shorter than
+    the block) in several."""
+    rng = np.random.default_rng(hits + history)
+    nt, nsub, nchan = history + 4200, 8, 16
+    x = rng.normal(1000.0, 30.0, (nt, nsub * nchan))
+    for t in history + 10 + rng.choice(nt - history - 10, hits, replace=False):
+        c = rng.choice(nsub * nchan, nsub * nchan // 5, replace=False)
+        x[t, c] += rng.uniform(0.0, 2500.0, c.size)
+    x *= np.linspace(1.0, 1.05, nt)[:, None]
+    bp = make_bp_text(nsub * nchan, START, WIDTH, 1000.0, 50.0)
+    _run(pv, oracle, cuda, x.astype(np.float32).reshape(nt, nsub, 1, nchan), (history,), bp, history)

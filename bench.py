@@ -707,7 +707,7 @@ def run_batch(args, cfgs, workload):
                                % (nsm, peak_src),
                 "per_unit": "one FP32 add per DM-trial*channel*sample (%d per launch)" % units_step,
                 "kernel_ms": st["dedisperse"]}
-    roofline_chan = {"kernel": "chan_stokes_i_kernel", "bound": "hbm", "achieved": chan_gbs,
+    roofline_chan = {"kernel": "chan_stokes_seg_kernel", "bound": "hbm", "achieved": chan_gbs,
                      "peak": hbm, "unit": "GB/s", "frac": chan_gbs / hbm,
                      "per_unit": "int16 voltages in (%d B) + float filterbank out (%d B) per step"
                                  % (in_bytes, fb_bytes),
@@ -738,7 +738,7 @@ def run_batch(args, cfgs, workload):
                                    "beams of more than 1024 channels on clusters of 128-thread CTAs"
                                    if args.rfi_cluster8 else (
                                        "one CTA per beam up to 4096 channels, else a cluster of 4 CTAs"
-                                       if args.rfi_cluster4 or args.unpipelined else "one CTA per beam")),
+                                       if args.rfi_cluster4 else "in blocks of 2048 spectra")),
                        "parallelism": "replicas" if world > 1 else "one GPU, all beams batched"},
             "e2e": {"value": e2e_value, "unit": "DM-trial*chan*samples/s",
                     "h2d_bytes_per_step": in_bytes, "d2h_bytes_per_step": d2h,
@@ -760,10 +760,9 @@ def run_batch(args, cfgs, workload):
                               "ring_write_wall": st["ring_write"], "dedisperse": st["dedisperse"],
                               "analyse": st["analyse"],
                               "what": "mean over the timed steps of the CUDA-event intervals at the stage "
-                                      "boundaries on each stage's stream; pipelined, rfi_wall and "
-                                      "ring_write_wall include the waits of those streams for SMs the "
-                                      "concurrent dedispersion holds (the kernels alone: the launch list "
-                                      "in profiles/)"},
+                                      "boundaries on each stage's stream; pipelined with walked "
+                                      "clippers, rfi_wall and ring_write_wall include the waits of those "
+                                      "streams for SMs the concurrent dedispersion holds"},
             "tiles": {k: tiles[k] for k in ("variant", "time_tile", "chan_per_stage", "stages",
                                              "slot", "tiles", "ctas", "tune_ms", "graph_kernels")},
             "latency_ms": {"p50": float(np.percentile(lat_ms, 50)),

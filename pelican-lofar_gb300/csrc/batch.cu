@@ -2,28 +2,31 @@
 // channel counts, trial counts and delay ranges advance one chunk per step,
 // each stage of all beams in as few launches as the kernels allow:
 //
-//   K1  chan_stokes_i_kernel   one launch per channels-per-subband class
-//   K2  rfi_batch_kernel       one CTA per beam, one launch per channel count
+//   K1  chan_stokes_seg_kernel one launch per channels-per-subband class
+//   K2  the clipper in blocks  three to five launches per block of 2048 spectra
+//                              and channel count (rfi_batch_kernel, one CTA or
+//                              cluster per beam, where the clipper is walked)
 //   A8  ring_write_batch_kernel one launch
 //   K4  dedisperse_batch_kernel one persistent launch over every beam's tiles,
 //                              DM x time tile shape chosen by the autotuner
 //   K5  analyser               per beam (count, scan, emit)
 //
-// Pipelined mode (PV_BATCH_PIPELINED) splits a step into two concurrent
-// branches after the channeliser: clip and ring-write chunk k, and meanwhile
-// dedisperse and search window k-lag-1 (complete since the previous step).
-// The clippers run one CTA per beam, so the persistent dedispersion launch
-// fills the SMs they leave idle; every ring holds one more chunk so that the
-// branches never touch the same ring positions, and a window's events come
-// one step later.
+// Pipelined mode (PV_BATCH_PIPELINED): a step clips and ring-writes chunk k
+// and dedisperses and searches window k-lag-1, complete since the previous
+// step.  Every ring holds one more chunk so that the two never touch the same
+// ring positions, and a window's events come one step later.  Clippers in
+// blocks fill the GPU and come first; walked ones (one CTA per beam) run
+// beside the persistent dedispersion launch, which then fills the SMs they
+// leave idle.
 // Every launch reads the chunk index from a device step counter that the
 // step's last kernel advances, so one captured CUDA graph replays every
 // step unchanged.  Inputs and event outputs are double buffered by step
 // parity: the host copies the next step's voltages (on the batch's copy
 // stream) while the current step computes, and each step's events land in
-// host-mapped pinned memory, readable while the next step runs.  The chain of each beam is the pv_beam chain: the same
-// state layout (tap history, RFI state, delay ring) and the same arithmetic,
-// so a beam's events in the batch equal its events run alone.
+// host-mapped pinned memory, readable while the next step runs.  The chain of
+// each beam is the pv_beam chain: the same state layout (tap history, RFI
+// state, delay ring) and the same arithmetic, so a beam's events in the batch
+// equal its events run alone.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -1299,12 +1299,22 @@ int dedisperse_device(float* out, long long out_stride, const float* in, long lo
     }
     DedispArgs a{out, out_stride, in, row_stride, row_len, ring_len, t_base % std::max(ring_len, 1LL),
                  d_dmshift, nchan, nout, tdms, start, step, 0, wait_ns(), 0};
+    // the plain kernels: the widest trial tile whose two buffers fit shared memory
+    const auto fits16 = [&] { return (size_t)2 * 4 * (1024 + spread(16)) * 4 <= 200 * 1024; };
+    const auto fits8 = [&] { return (size_t)2 * 4 * (1024 + spread(8)) * 4 <= 220 * 1024; };
+    const auto fits4 = [&] { return (size_t)2 * 2 * (512 + spread(4)) * 4 <= 220 * 1024; };
     // Rows whose 16-byte units bulk copies can fetch go through the pipeline.
     const bool aligned = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
     const bool ring = ring_len > 0 && ring_len % 4 == 0 && row_stride % 4 == 0;
     if (status && aligned && (ring || ring_len == 0) && getenv("PV_DEDISP_V1") == nullptr) {
         if (ring) a.stall = take_stall();
-        const int v = tma_tile(tdms, nout, ring_len, spread);
+        // A ring that the plain kernels refuse (shorter than their tile's span) stays refused where a
+        // narrower tile's span would fit.
+        const bool plain_ok = ring_len == 0 || [&] {
+            const int tt = fits16() || fits8() ? 1024 : 512, dms = fits16() ? 16 : fits8() ? 8 : fits4() ? 4 : 1;
+            return ring_len >= (long long)std::min(tt, nout) + spread(dms);
+        }();
+        const int v = plain_ok ? tma_tile(tdms, nout, ring_len, spread) : -1;
         if (v >= 0) {
             const int sp = spread(kTmaTiles[v].dms);
             if (v == 0) return launch_dedisperse_tma<16, 32, 8, 2>(a, sp, status, s);
@@ -1315,17 +1325,10 @@ int dedisperse_device(float* out, long long out_stride, const float* in, long lo
             return launch_dedisperse_pair<4, 8, 2>(a, sp, status, s);
         }
     }
-    const int spread16 = spread(16);
-    if ((size_t)2 * 4 * (1024 + spread16) * 4 <= 200 * 1024)
-        return launch_dedisperse<16, 32, 4>(a, spread16, s);
-    const int spread8 = spread(8);
-    if ((size_t)2 * 4 * (1024 + spread8) * 4 <= 220 * 1024)
-        return launch_dedisperse<8, 32, 4>(a, spread8, s);
-    const int spread4 = spread(4);
-    if ((size_t)2 * 2 * (512 + spread4) * 4 <= 220 * 1024)
-        return launch_dedisperse<4, 16, 2>(a, spread4, s);
-    const int spread1 = spread(1);
-    return launch_dedisperse<1, 16, 1>(a, spread1, s);
+    if (fits16()) return launch_dedisperse<16, 32, 4>(a, spread(16), s);
+    if (fits8()) return launch_dedisperse<8, 32, 4>(a, spread(8), s);
+    if (fits4()) return launch_dedisperse<4, 16, 2>(a, spread(4), s);
+    return launch_dedisperse<1, 16, 1>(a, spread(1), s);
 }
 
 }  // namespace pv

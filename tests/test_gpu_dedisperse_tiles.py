@@ -119,3 +119,13 @@ def test_trial_pairs(pv, oracle, cuda, case, ring):
     got = plan.run(xd, nout, ring_len=width if ring else 0, t_base=base)
     assert np.array_equal(got.cpu().numpy(), want)
     assert plan.status() == 0
+
+
+def test_short_ring_stays_refused(pv, cuda):
+    """A ring shorter than a wide tile's span is an error whichever tile would be faster."""
+    import torch
+    k, _ = pv.dm_shifts(150.0, -0.05, 33)
+    plan = pv.DedispPlan(k, 64, 0.0, 20000.0)
+    x = torch.zeros(33, 1600, device=cuda)
+    with pytest.raises(Exception):
+        plan.run(x, 1000, ring_len=1600)

@@ -365,11 +365,12 @@ __device__ __forceinline__ void tma_producer(const DedispArgs& a, const Pipe<CS,
             mbar_wait_warp(&full[st % ST], (unsigned)(st / ST) & 1u, pv::kDrainWaitNs);
 }
 
-template <int DMS, int R, int CS, int ST>
-__global__ void __launch_bounds__((DMS + 1) * 32)
+template <int DMS, int PARTS, int R, int CS, int ST>
+__global__ void __launch_bounds__((DMS * PARTS + 1) * 32)
 dedisperse_tma_kernel(const DedispArgs a, int* __restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    constexpr int TT = 32 * R;
+    constexpr int TT = 32 * R * PARTS;
+    constexpr int NW = DMS * PARTS;
     Pipe<CS, ST> pipe(smem_raw, a.slot);
     const float* slots = pipe.slots;
     const int* meta_off = pipe.meta_off;
@@ -381,15 +382,16 @@ dedisperse_tma_kernel(const DedispArgs a, int* __restrict__ status) {
     const int d0 = blockIdx.y * DMS;
     const int d_last = min(d0 + DMS, a.tdms) - 1;
     const int nstages = (a.nchan + CS - 1) / CS;
-    if (!pipe.start(DMS, status)) return;
-    if (warp == DMS) {
+    if (!pipe.start(NW, status)) return;
+    if (warp == NW) {
         tma_producer<TT, CS, ST>(a, pipe, t0, pv_trial_value(d0, a.start, a.step),
                                  pv_trial_value(d_last, a.start, a.step), status, lane);
         return;
     }
 
     // ---------------- consumers ----------------
-    const int d = d0 + warp;
+    const int d = d0 + warp % DMS;
+    const int first = warp / DMS * 32 * R + lane;  // the lane's first sample in the tile
     const bool active = d <= d_last;
     const float dv = pv_trial_value(d, a.start, a.step);
     float acc[R];
@@ -411,7 +413,7 @@ dedisperse_tma_kernel(const DedispArgs a, int* __restrict__ status) {
                 lane < c_end ? min(pv_shift(meta_k[b * CS + lane], dv) - meta_off[b * CS + lane], a.slot - TT) : 0;
             for (int j = 0; j < c_end; ++j) {
                 const int off = __shfl_sync(0xffffffffu, my_off, j);
-                const float* row = slots + (size_t)(b * CS + j) * a.slot + off + lane;
+                const float* row = slots + (size_t)(b * CS + j) * a.slot + off + first;
 #pragma unroll
                 for (int r = 0; r < R; ++r) acc[r] = __fadd_rn(acc[r], row[32 * r]);
             }
@@ -423,7 +425,7 @@ dedisperse_tma_kernel(const DedispArgs a, int* __restrict__ status) {
         float* o = a.out + (long long)d * a.out_stride;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const long long t = t0 + lane + 32 * r;
+            const long long t = t0 + first + 32 * r;
             if (t < a.nout) o[t] = acc[r];
         }
     }
@@ -1161,17 +1163,17 @@ int launch_dedisperse(DedispArgs a, int spread, cudaStream_t s) {
     return pv::check_launch("dedisperse_kernel");
 }
 
-template <int DMS, int R, int CS, int ST>
+template <int DMS, int PARTS, int R, int CS, int ST>
 int launch_dedisperse_tma(DedispArgs a, int spread, int* status, cudaStream_t s) {
-    constexpr int TT = 32 * R;
+    constexpr int TT = 32 * R * PARTS;
     a.slot = (TT + spread + 8 + 3) & ~3;
     const size_t smem = (size_t)ST * CS * a.slot * sizeof(float) + (size_t)ST * CS * 8 + 8 +
                         (size_t)2 * ST * sizeof(uint64_t);
-    auto kern = dedisperse_tma_kernel<DMS, R, CS, ST>;
+    auto kern = dedisperse_tma_kernel<DMS, PARTS, R, CS, ST>;
     PV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
             "cudaFuncSetAttribute(dedisperse_tma)");
     dim3 grid((unsigned)pv::ceil_div<long long>(a.nout, TT), (unsigned)pv::ceil_div(a.tdms, DMS));
-    kern<<<grid, (DMS + 1) * 32, smem, s>>>(a, status);
+    kern<<<grid, (DMS * PARTS + 1) * 32, smem, s>>>(a, status);
     return pv::check_launch("dedisperse_tma_kernel");
 }
 
@@ -1230,6 +1232,43 @@ constexpr TmaTile kTmaTiles[] = {{16, 1024, 8, 2, 1.0f, 0.0f, 0},  {16, 1024, 2,
                                  {8, 1024, 8, 2, 0.95f, 0.0f, 0},  {8, 256, 16, 2, 0.93f, 0.0f, 0},
                                  {14, 1056, 8, 2, 1.27f, 0.02f, 2}, {8, 1056, 8, 2, 1.28f, 0.03f, 3}};
 constexpr int kOneTrialTiles = 4, kTiles = 6;
+// Narrow tiles of the one-trial kernel, for calls of few trials or samples and
+// for delays that differ by hundreds of samples from one trial to the next
+// (whose wide tiles do not fit shared memory): trials x parts x samples a
+// lane, channels per stage, stages.  32-channel stages halve the waits of the
+// small ones.  us of the best wide tile / the narrow one taken (0: none fits,
+// the plain kernel's time), by the largest difference between two trials:
+//   100 trials x 1024 channels x 3000, 0        88    66  4 x 256
+//   64 x 256 x 512, 22                          32    26  1 x 256
+//   200 x 256 x 3000, 156                       62    42  2 x 1024
+//   60 x 500 x 9000, 754                       405 0  74  2 x 1024
+//   128 x 2000 x 3000, 761                    1677 0 267  2 x 1024
+//   16 x 500 x 16000, 1976                     387 0  62  1 x 1024
+//   20 x 4096 x 4000, 5089                    2032 0 202  1 x 256
+struct NarrowTile {
+    int dms, parts, r, cs, st;
+    constexpr int tt() const { return 32 * parts * r; }
+};
+constexpr NarrowTile kNarrowTiles[] = {{8, 1, 8, 32, 2}, {4, 1, 8, 32, 2}, {4, 4, 8, 8, 2},
+                                       {2, 4, 8, 8, 2},  {1, 4, 8, 8, 3},  {1, 2, 4, 32, 2}};
+
+// SM cycles per channel of the busiest SM: rounds of the resident CTAs, each
+// stage at the larger of its shared-memory reads, its copies through L2 and a
+// stage's latency over the stages in flight.  The constants are a fit to 340
+// launches of 25 tiles on 37 shapes (one standard deviation 20 %).
+inline double pipe_cycles(const NarrowTile& t, int sp, int tdms, int nout) {
+    const double copied = 4.0 * (t.tt() + 0.5 * sp) / 38.0;
+    const size_t smem = tma_smem(t.st, t.cs, (t.tt() + sp + 8 + 3) & ~3) + 1024;
+    const int threads = 32 * (t.dms * t.parts + 1);
+    const long long held = std::max(1LL, std::min({(long long)(227 * 1024 / smem), 65536LL / (threads * (40 + t.r)),
+                                                   2048LL / threads}));
+    const long long ctas = ceil_div((long long)ceil_div(tdms, t.dms) * ceil_div(nout, t.tt()), (long long)sm_count());
+    const auto round = [&](long long q) {
+        return std::max({q * t.dms * t.parts * (t.r + 2) / 0.95, q * copied,
+                         (2250.0 / t.cs + 6.9 * (t.r + 3.8) + copied) / t.st});
+    };
+    return ctas / held * round(held) + (ctas % held ? round(ctas % held) : 0.0);
+}
 
 // The tile with the least expected time, -1 if none fits: the busiest SM's
 // share of the adds, at a rate that falls where a tile copies more than 0.55
@@ -1265,7 +1304,7 @@ int tma_tile(int tdms, int nout, long long ring_len, F spread) {
             best_t = time;
         }
     }
-    const double diff = spread(8) / 7.0;
+    const double diff = (double)spread(8) / std::max(1, std::min(8, tdms) - 1);
     for (int v = kOneTrialTiles; v < kTiles && best >= 0; ++v) {
         const TmaTile& t = kTmaTiles[v];
         const double rate = t.rate - t.slope * 0.5 * diff;
@@ -1281,6 +1320,25 @@ int tma_tile(int tdms, int nout, long long ring_len, F spread) {
             best = v;
             best_t = time;
         }
+    }
+    if (best >= kOneTrialTiles) return best;
+    // a narrow one where it is expected to gain more than its estimate errs among tiles that measured alike
+    double now = 1e30;
+    if (best >= 0) {
+        const TmaTile& t = kTmaTiles[best];
+        now = 0.93 * pipe_cycles({t.dms, 1, t.tt / 32, t.cs, t.st}, spread(t.dms), tdms, nout);
+    }
+    for (int v = 0; v < (int)(sizeof(kNarrowTiles) / sizeof(kNarrowTiles[0])); ++v) {
+        const NarrowTile& t = kNarrowTiles[v];
+        if (ceil_div(tdms, t.dms) > 65535) continue;
+        const double cycles = pipe_cycles(t, (int)(diff * (t.dms - 1)), tdms, nout);
+        if (cycles >= now) continue;
+        const int sp = t.dms == 1 ? 0 : spread(t.dms);
+        if (tma_smem(t.st, t.cs, (t.tt() + sp + 8 + 3) & ~3) > 220 * 1024 ||
+            (ring_len > 0 && ring_len < (long long)std::min(t.tt(), nout) + sp + 8))
+            continue;
+        best = kTiles + v;
+        now = cycles;
     }
     return best;
 }
@@ -1316,13 +1374,19 @@ int dedisperse_device(float* out, long long out_stride, const float* in, long lo
         }();
         const int v = plain_ok ? tma_tile(tdms, nout, ring_len, spread) : -1;
         if (v >= 0) {
-            const int sp = spread(kTmaTiles[v].dms);
-            if (v == 0) return launch_dedisperse_tma<16, 32, 8, 2>(a, sp, status, s);
-            if (v == 1) return launch_dedisperse_tma<16, 32, 2, 4>(a, sp, status, s);
-            if (v == 2) return launch_dedisperse_tma<8, 32, 8, 2>(a, sp, status, s);
-            if (v == 3) return launch_dedisperse_tma<8, 8, 16, 2>(a, sp, status, s);
+            const int sp = spread(v < kTiles ? kTmaTiles[v].dms : kNarrowTiles[v - kTiles].dms);
+            if (v == 0) return launch_dedisperse_tma<16, 1, 32, 8, 2>(a, sp, status, s);
+            if (v == 1) return launch_dedisperse_tma<16, 1, 32, 2, 4>(a, sp, status, s);
+            if (v == 2) return launch_dedisperse_tma<8, 1, 32, 8, 2>(a, sp, status, s);
+            if (v == 3) return launch_dedisperse_tma<8, 1, 8, 16, 2>(a, sp, status, s);
             if (v == 4) return launch_dedisperse_pair<7, 8, 2>(a, sp, status, s);
-            return launch_dedisperse_pair<4, 8, 2>(a, sp, status, s);
+            if (v == 5) return launch_dedisperse_pair<4, 8, 2>(a, sp, status, s);
+            if (v == 6) return launch_dedisperse_tma<8, 1, 8, 32, 2>(a, sp, status, s);
+            if (v == 7) return launch_dedisperse_tma<4, 1, 8, 32, 2>(a, sp, status, s);
+            if (v == 8) return launch_dedisperse_tma<4, 4, 8, 8, 2>(a, sp, status, s);
+            if (v == 9) return launch_dedisperse_tma<2, 4, 8, 8, 2>(a, sp, status, s);
+            if (v == 10) return launch_dedisperse_tma<1, 4, 8, 8, 3>(a, sp, status, s);
+            return launch_dedisperse_tma<1, 2, 4, 32, 2>(a, sp, status, s);
         }
     }
     if (fits16()) return launch_dedisperse<16, 32, 4>(a, spread(16), s);

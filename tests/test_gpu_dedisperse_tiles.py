@@ -121,6 +121,33 @@ def test_trial_pairs(pv, oracle, cuda, case, ring):
     assert plan.status() == 0
 
 
+NARROW_CASES = [
+    # few trials or samples, or delays far apart from one trial to the next (2.4e-4 per unit of
+    # the step and channel at the lowest): 8 x 256 and 4 x 256 in 32-channel stages, 4, 2 and
+    # 1 x 1024, 1 x 256; fewer trials than the eight that the rule's spread is taken of
+    (70, 512, 1025, 150.0, -0.05, 600.0),
+    (65, 99, 3000, 150.0, -0.05, 5.0),
+    (33, 64, 513, 150.0, -0.05, 5000.0),
+    (33, 200, 3000, 150.0, -0.05, 40000.0),
+    (31, 61, 9001, 150.0, -0.05, 190000.0),
+    (33, 16, 16001, 150.0, -0.05, 500000.0),
+    (40, 20, 1000, 150.0, -0.05, 1000000.0),
+    (33, 7, 300, 150.0, -0.05, 5000.0),
+    (5, 1, 255, 150.0, -0.05, 5000.0),
+]
+
+
+@pytest.mark.parametrize("ring", [False, True])
+@pytest.mark.parametrize("case", NARROW_CASES)
+def test_narrow_tiles(pv, oracle, cuda, case, ring):
+    test_trial_pairs(pv, oracle, cuda, case, ring)
+
+
+@pytest.mark.parametrize("case", NARROW_CASES[1:7])
+def test_narrow_tiles_past_the_rows_end(pv, oracle, cuda, case):
+    test_rows_that_end_early(pv, oracle, cuda, case, 700)
+
+
 def test_short_ring_stays_refused(pv, cuda):
     """A ring shorter than a wide tile's span is an error whichever tile would be faster."""
     import torch

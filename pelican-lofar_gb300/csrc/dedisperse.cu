@@ -1280,9 +1280,9 @@ inline double pipe_cycles(const NarrowTile& t, int sp, int tdms, int nout) {
 template <typename F>
 int tma_tile(int tdms, int nout, long long ring_len, F spread) {
     const auto smem_of = [](const TmaTile& t, int sp) { return tma_smem(t.st, t.cs, (t.tt + sp + 8 + 3) & ~3); };
-    // two stages fit, and every copy (span + 16-byte rounding) in one ring turn
+    // two stages fit, every copy (span + 16-byte rounding) in one ring turn, and the tiles in a grid
     const auto fits = [&](const TmaTile& t, int sp) {
-        return smem_of(t, sp) <= 220 * 1024 &&
+        return smem_of(t, sp) <= 220 * 1024 && ceil_div(tdms, t.dms) <= 65535 &&
                (ring_len <= 0 || ring_len >= (long long)std::min(t.tt, nout) + sp + 8);
     };
     const auto time_of = [&](const TmaTile& t, int sp, double rate, double busiest) {

@@ -1305,10 +1305,11 @@ int tma_tile(int tdms, int nout, long long ring_len, F spread) {
         }
     }
     const double diff = (double)spread(8) / std::max(1, std::min(8, tdms) - 1);
+    const auto guess = [&](int dms) { return (int)std::min(1e8, diff * (dms - 1)); };
     for (int v = kOneTrialTiles; v < kTiles && best >= 0; ++v) {
         const TmaTile& t = kTmaTiles[v];
         const double rate = t.rate - t.slope * 0.5 * diff;
-        const int sp = (int)(diff * (t.dms - 1));  // exact only where it could win: the host pays for each spread
+        const int sp = guess(t.dms);  // exact only where it could win: the host pays for each spread
         if (rate <= 0.5) continue;
         const double held = std::min(t.resident, (int)(227 * 1024 / (smem_of(t, sp) + 1024)));
         if (held < 1.0) continue;
@@ -1331,7 +1332,7 @@ int tma_tile(int tdms, int nout, long long ring_len, F spread) {
     for (int v = 0; v < (int)(sizeof(kNarrowTiles) / sizeof(kNarrowTiles[0])); ++v) {
         const NarrowTile& t = kNarrowTiles[v];
         if (ceil_div(tdms, t.dms) > 65535) continue;
-        const double cycles = pipe_cycles(t, (int)(diff * (t.dms - 1)), tdms, nout);
+        const double cycles = pipe_cycles(t, guess(t.dms), tdms, nout);
         if (cycles >= now) continue;
         const int sp = t.dms == 1 ? 0 : spread(t.dms);
         if (tma_smem(t.st, t.cs, (t.tt() + sp + 8 + 3) & ~3) > 220 * 1024 ||

@@ -43,15 +43,19 @@ long long pv_kernel_launches(void);
  * runs out makes the kernel record PV_ERR_TIMEOUT, wait for its own copies
  * in flight (up to 0.5 s) and return; the launch's other CTAs stop, and the
  * status reaches the caller through pv_dedisp_plan_status, pv_beam_events or
- * pv_batch_events.  A CUDA graph keeps the limit it was captured with.
+ * pv_batch_events.  On linear rows (pv_dedisperse, pv_dedisperse_ex,
+ * pv_dedisp_plan_run with ring_len 0) there is nothing to report: the warps
+ * whose wait runs out read their samples from global memory instead, and the
+ * outputs are the same.  A CUDA graph keeps the limit it was captured with.
  * Returns the previous limit.  No counterpart in the reference, whose
  * GPU_Job reports failures as GPU_Job::Failed (lib/src/GPU_Manager.cpp). */
 long long pv_set_wait_limit(long long ns);
 /* Failure-path test hook: the next n pipelined dedispersion launches (single
- * beam, plan or pv_dedisperse on ring rows) withhold the copies of their
- * first channel stage in every CTA, so the consumers' wait on that stage
- * can only end at the wait limit.  Nothing faults or hangs: the kernel
- * records PV_ERR_TIMEOUT and returns, as for a copy that never lands.
+ * beam, plan or pv_dedisperse) withhold the copies of their first channel
+ * stage in every CTA, so the consumers' wait on that stage can only end at
+ * the wait limit.  Nothing faults or hangs: on ring rows the kernel records
+ * PV_ERR_TIMEOUT and returns, on linear rows it does without the copies, as
+ * for a copy that never lands.
  * Returns the previous count. */
 int pv_stall_next_launches(int n);
 /* cudaMemcpyAsync with cudaMemcpyDefault (host or device pointers). */

@@ -184,7 +184,9 @@ dedisperse_kernel(const DedispArgs a) {
 // memory in channel order and release the buffer on "empty".  Span starts are
 // rounded down to 16 bytes; the rounding offset is folded into the per-channel
 // offset table the producer writes beside the data.  Every wait is bounded by
-// %globaltimer; a wait that gives up records PV_ERR_TIMEOUT in *status.
+// %globaltimer.  Ring rows: a wait that gives up records PV_ERR_TIMEOUT in
+// *status.  Linear rows have no status (null): a consumer warp that gives up
+// adds its samples from global memory instead (direct_sums).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
     return (unsigned)__cvta_generic_to_shared(p);
@@ -256,7 +258,7 @@ struct Pipe {
     __device__ __forceinline__ bool start(int consumers, const int* status) {
         __shared__ int s_abort;
         if (threadIdx.x == 0) {
-            s_abort = *(volatile const int*)status;
+            s_abort = status ? *(volatile const int*)status : 0;
             for (int b = 0; b < ST; ++b) {
                 mbar_init(&full[b], 1);
                 mbar_init(&empty[b], (unsigned)consumers);
@@ -293,7 +295,7 @@ __device__ __forceinline__ void tma_producer(const DedispArgs& a, const Pipe<CS,
         const int b = st % ST;
         const unsigned round = (unsigned)(st / ST);
         if (!mbar_wait_warp(&empty[b], (round & 1u) ^ 1u, a.wait_ns)) {
-            if (lane == 0) atomicExch(status, PV_ERR_TIMEOUT);
+            if (lane == 0 && status) atomicExch(status, PV_ERR_TIMEOUT);
             ok = false;
             break;
         }
@@ -365,9 +367,27 @@ __device__ __forceinline__ void tma_producer(const DedispArgs& a, const Pipe<CS,
             mbar_wait_warp(&full[st % ST], (unsigned)(st / ST) & 1u, pv::kDrainWaitNs);
 }
 
+// Linear rows without the pipeline: one warp writes samples [t, end) of trial
+// d, the same sums read from global memory.  For a consumer whose wait gave
+// up, so that no call on linear rows can fail after its launch.
+__device__ __noinline__ void direct_sums(const DedispArgs& a, int d, long long t, long long end) {
+    const int lane = threadIdx.x & 31;
+    const float dv = pv_trial_value(d, a.start, a.step);
+    float* o = a.out + (long long)d * a.out_stride;
+    for (t += lane; t < end; t += 32) {
+        float acc = 0.0f;
+#pragma unroll 1
+        for (int c = 0; c < a.nchan; ++c) {
+            const long long g = (long long)c * a.row_stride + t + pv_shift(a.dmshift[c], dv);
+            acc = __fadd_rn(acc, g < linear_end(a, c) ? a.in[g] : 0.0f);
+        }
+        o[t] = acc;
+    }
+}
+
 template <int DMS, int PARTS, int R, int CS, int ST>
 __global__ void __launch_bounds__((DMS * PARTS + 1) * 32)
-dedisperse_tma_kernel(const DedispArgs a, int* __restrict__ status) {
+dedisperse_tma_kernel(const __grid_constant__ DedispArgs a, int* __restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int TT = 32 * R * PARTS;
     constexpr int NW = DMS * PARTS;
@@ -397,13 +417,16 @@ dedisperse_tma_kernel(const DedispArgs a, int* __restrict__ status) {
     float acc[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) acc[r] = 0.0f;
-    bool ok = true;
     for (int st = 0; st < nstages; ++st) {
         const int b = st % ST;
         if (!mbar_wait_warp(&full[b], (unsigned)(st / ST) & 1u, a.wait_ns)) {
-            if (lane == 0) atomicExch(status, PV_ERR_TIMEOUT);
-            ok = false;
-            break;
+            if (a.ring_len > 0) {
+                if (lane == 0) atomicExch(status, PV_ERR_TIMEOUT);
+            } else if (active) {
+                const long long t = t0 + first - lane;
+                direct_sums(a, d, t, min(t + 32 * R, (long long)a.nout));
+            }
+            return;
         }
         if (active) {
             const int c_end = min(CS, a.nchan - st * CS);
@@ -421,7 +444,7 @@ dedisperse_tma_kernel(const DedispArgs a, int* __restrict__ status) {
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[b]);
     }
-    if (ok && active) {
+    if (active) {
         float* o = a.out + (long long)d * a.out_stride;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -943,7 +966,7 @@ __device__ __forceinline__ void pair_dispatch(const float* __restrict__ row, int
 // channels x 8192 samples 979 -> 833 us, the tile rule below has more.
 template <int PAIRS, int CS, int ST>
 __global__ void __launch_bounds__((PAIRS + 1) * 32, 16 / (PAIRS + 1))
-dedisperse_tma_pair_kernel(const DedispArgs a, int* __restrict__ status) {
+dedisperse_tma_pair_kernel(const __grid_constant__ DedispArgs a, int* __restrict__ status) {
     constexpr int TT = 32 * kPairS;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     Pipe<CS, ST> pipe(smem_raw, a.slot);
@@ -969,7 +992,12 @@ dedisperse_tma_pair_kernel(const DedispArgs a, int* __restrict__ status) {
     for (int st = 0; st < nstages; ++st) {
         const int b = st % ST;
         if (!mbar_wait_warp(&pipe.full[b], (unsigned)(st / ST) & 1u, a.wait_ns)) {
-            if (lane == 0) atomicExch(status, PV_ERR_TIMEOUT);
+            if (a.ring_len > 0) {
+                if (lane == 0) atomicExch(status, PV_ERR_TIMEOUT);
+            } else {
+                for (int d = da; d <= min(da + 1, d_last); ++d)
+                    direct_sums(a, d, t0, min(t0 + TT, (long long)a.nout));
+            }
             return;
         }
         if (act_a) {
@@ -1365,8 +1393,8 @@ int dedisperse_device(float* out, long long out_stride, const float* in, long lo
     // Rows whose 16-byte units bulk copies can fetch go through the pipeline.
     const bool aligned = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
     const bool ring = ring_len > 0 && ring_len % 4 == 0 && row_stride % 4 == 0;
-    if (status && aligned && (ring || ring_len == 0) && getenv("PV_DEDISP_V1") == nullptr) {
-        if (ring) a.stall = take_stall();
+    if (ring_len == 0) status = nullptr;  // direct_sums: nothing to report
+    if (aligned && (ring ? status != nullptr : ring_len == 0) && getenv("PV_DEDISP_V1") == nullptr) {
         // A ring that the plain kernels refuse (shorter than their tile's span) stays refused where a
         // narrower tile's span would fit.
         const bool plain_ok = ring_len == 0 || [&] {
@@ -1375,6 +1403,7 @@ int dedisperse_device(float* out, long long out_stride, const float* in, long lo
         }();
         const int v = plain_ok ? tma_tile(tdms, nout, ring_len, spread) : -1;
         if (v >= 0) {
+            a.stall = take_stall();
             const int sp = spread(v < kTiles ? kTmaTiles[v].dms : kNarrowTiles[v - kTiles].dms);
             if (v == 0) return launch_dedisperse_tma<16, 1, 32, 8, 2>(a, sp, status, s);
             if (v == 1) return launch_dedisperse_tma<16, 1, 32, 2, 4>(a, sp, status, s);
@@ -1797,31 +1826,6 @@ extern "C" int pv_delay_table(int* d_shifts, const float* d_dmshift, int nchan, 
 
 namespace {
 
-// Status words of pv_dedisperse_ex launches, one per call in turn, per device:
-// a call reports (and clears) what an earlier one recorded.
-constexpr int kExWords = 256;
-struct ExStatus {
-    int* words = nullptr;
-    unsigned next = 0;
-};
-std::mutex g_ex_mutex;
-std::map<int, ExStatus> g_ex;
-
-int ex_status(int** all, int** mine) {
-    int dev = 0;
-    PV_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
-    std::lock_guard<std::mutex> lk(g_ex_mutex);
-    ExStatus& e = g_ex[dev];
-    if (!e.words) {
-        PV_CUDA(cudaMalloc(&e.words, sizeof(int) * kExWords), "allocate dedispersion status");
-        PV_CUDA(cudaMemset(e.words, 0, sizeof(int) * kExWords), "clear dedispersion status");
-        PV_CUDA(cudaStreamSynchronize(cudaStreamLegacy), "clear dedispersion status");
-    }
-    *all = e.words;
-    *mine = e.words + e.next++ % kExWords;
-    return PV_OK;
-}
-
 // A thread's page-locked staging (reads from it need no copy by the driver).
 struct Staging {
     void* p = nullptr;
@@ -1857,22 +1861,12 @@ extern "C" int pv_dedisperse_ex(float* d_out, long long out_stride, const float*
     if (tdms == 0 || nout == 0) return PV_OK;
     std::vector<float> h(nchans);
     cudaStream_t s = pv::as_stream(stream);
-    int *words = nullptr, *status = nullptr;
-    PV_TRY(ex_status(&words, &status));
     void* staging = nullptr;
-    PV_TRY(t_staging.get(sizeof(float) * nchans + sizeof(int) * kExWords, &staging));
-    int* seen = reinterpret_cast<int*>(static_cast<float*>(staging) + nchans);
+    PV_TRY(t_staging.get(sizeof(float) * nchans, &staging));
     PV_CUDA(cudaMemcpyAsync(staging, d_dmshift, sizeof(float) * nchans, cudaMemcpyDeviceToHost, s),
             "copy dmshift");
-    PV_CUDA(cudaMemcpyAsync(seen, words, sizeof(int) * kExWords, cudaMemcpyDeviceToHost, s), "read status");
     PV_CUDA(cudaStreamSynchronize(s), "synchronise");
     std::copy(static_cast<float*>(staging), static_cast<float*>(staging) + nchans, h.begin());
-    for (int i = 0; i < kExWords; ++i)
-        if (seen[i] != PV_OK) {
-            PV_CUDA(cudaMemsetAsync(words, 0, sizeof(int) * kExWords, s), "clear status");
-            pv::set_error("pv_dedisperse_ex: a pipeline wait of an earlier call gave up (status %d)", seen[i]);
-            return seen[i];
-        }
     // Every delay must be a finite, non-negative sample count: the tiles
     // address shared memory and the input relative to the first trial's delay.
     if (!(start_over_tsamp >= 0.0f) || !(step_over_tsamp >= 0.0f) ||
@@ -1901,7 +1895,7 @@ extern "C" int pv_dedisperse_ex(float* d_out, long long out_stride, const float*
         return spreads[dms] = delay_spread(h, tdms, dms, start_over_tsamp, step_over_tsamp);
     };
     return pv::dedisperse_device(d_out, out_stride, d_in, row_stride, row_len, 0, 0, nchans, nout, tdms, d_dmshift,
-                                 spread, start_over_tsamp, step_over_tsamp, s, status);
+                                 spread, start_over_tsamp, step_over_tsamp, s, nullptr);
 }
 
 extern "C" int pv_dedisperse(float* d_out, long long out_bytes, const float* d_in,

@@ -83,3 +83,39 @@ def test_beam_reports_timeout_and_other_beams_run(pv, oracle, cuda):
     ea, na, fa = good.events()
     eb, nb, fb = ref.events()
     assert na == nb and fa == fb == 0 and np.array_equal(ea, eb)
+
+
+@pytest.mark.parametrize("nchan,tdms,nout,step", [
+    (70, 300, 5003, 300.0),      # one trial per warp
+    (33, 9, 255, 400.0),         # a small call
+    (17, 1024, 8448, 5000.0),    # trial pairs
+])
+def test_linear_rows_settle_a_wait_that_runs_out(pv, oracle, cuda, nchan, tdms, nout, step):
+    """A call on linear rows has no status to report by: one whose copies
+    never land writes the same outputs, and neither it nor the next call
+    fails.  A plan's recorded ring failure does not touch its linear runs."""
+    import torch
+    k, _ = pv.dm_shifts(150.0, -0.05, nchan)
+    start, step = np.float32(1.5), np.float32(step)
+    ms = int(oracle.shift_table(k, tdms, start, step).max())
+    ring = (nout + ms + 1100 + 3) // 4 * 4
+    x = np.random.default_rng(nchan).standard_normal((nchan, ring)).astype(np.float32)
+    want = oracle.dedisperse(x, nout, tdms, k, start, step)
+    d, kd = torch.from_numpy(x).to(cuda), torch.from_numpy(k).to(cuda)
+    plan = pv.DedispPlan(k, tdms, float(start), float(step))
+    prev = pv.set_wait_limit(1000000)  # 1 ms
+    try:
+        for run in (lambda: pv.dedisperse(d, nout, tdms, kd, float(start), float(step)), lambda: plan.run(d, nout)):
+            pv.stall_next_launches(1)
+            assert np.array_equal(run().cpu().numpy(), want)
+            assert pv.stall_next_launches(0) == 0  # the hook was used by that launch
+            assert np.array_equal(run().cpu().numpy(), want)
+        assert plan.status() == 0
+        pv.stall_next_launches(1)
+        plan.run(d, nout, ring_len=ring, t_base=0)
+        torch.cuda.synchronize()
+        assert plan.status() == PV_ERR_TIMEOUT
+        assert np.array_equal(plan.run(d, nout).cpu().numpy(), want)
+    finally:
+        pv.stall_next_launches(0)
+        pv.set_wait_limit(prev)

@@ -228,7 +228,8 @@ int pv_analyse(const float* d_data, long long ld, int tdms, int nsamp, float thr
  * Every call on a device shares the one array, so calls that overlap on the
  * GPU (other streams, other host threads) race and corrupt each other's
  * results; serialise them.  Nothing in the array needs clearing between
- * calls: each call clears or writes everything it reads. */
+ * calls: a call writes what it reads, and leaves the one counter that it
+ * relies on at 0, also after an overlap. */
 #define PV_ANALYSE_NOALLOC_MAX_PAIRS (1 << 20)
 int pv_analyse_noalloc(const float* d_data, long long ld, int tdms, int nsamp, float threshold,
                        float rms, int bin_pow2, pv_event* d_events, long long cap,

@@ -88,7 +88,7 @@ constexpr int kCountThreads = 256;
 struct Tiles {
     long long* offset;  // [tiles] events before the tile's first
     int* count;         // [tiles]
-    unsigned* done;     // CTAs finished; 0 between calls
+    unsigned* done;     // CTAs of analyse_count finished; cleared by analyse_emit
 };
 
 // Runs in every CTA after it has stored its count: the last one to get here
@@ -123,7 +123,6 @@ __device__ __forceinline__ void finish_tiles(const Tiles& w, int ntiles, long lo
         at += __ldcg(w.count + i);
     }
     if (tid == kCountThreads - 1) *total = 1 + at;
-    if (tid == 0) *w.done = 0;
 }
 
 // Rows of 16-byte aligned samples, blocks of 8 to 256.  Lane l holds samples
@@ -222,15 +221,20 @@ __global__ void __launch_bounds__(kCountThreads) analyse_count(const float* __re
     finish_tiles(w, ntiles, total);
 }
 
-// CTA t writes tile t's events; CTA 0 the dummy event as well.
+// CTA t writes tile t's events; CTA 0 the dummy event as well.  CTA 0 clears
+// the counter of finished CTAs: after the count of its own call, so calls that
+// overlapped (which spoils their own results) leave it at 0 all the same.
 template <int P>
 __global__ void __launch_bounds__(kTilePairs) analyse_emit(const float* __restrict__ data, long long ld, int nblocks,
                                                            long long npairs, Thresholds thr, bool vec4, Tiles w,
                                                            pv_event* __restrict__ ev, long long cap) {
     __shared__ int wsum[kTilePairs / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (blockIdx.x == 0 && tid == 0 && cap > 0) ev[0] = pv_event{0, 0, 1.0f, 0.0f};
-    if (npairs == 0 || w.count[blockIdx.x] == 0) return;
+    if (blockIdx.x == 0 && tid == 0) {
+        *w.done = 0;
+        if (cap > 0) ev[0] = pv_event{0, 0, 1.0f, 0.0f};
+    }
+    if (w.count[blockIdx.x] == 0) return;
     const long long g = (long long)blockIdx.x * kTilePairs + tid;
     const int dm = (int)(g / nblocks), i = (int)(g % nblocks);
     const float* src = data + dm * ld + (long long)i * (1 << P);
@@ -310,7 +314,7 @@ int run_analyse(const float* data, long long ld, int tdms, int nsamp, const Thre
 namespace pv {
 
 // Scratch bytes the analyser needs for tdms x nsamp at 2^bin_pow2 blocks.  It
-// has to be cleared once; every call leaves its counter at 0.
+// has to be cleared once; every call clears its counter at its end.
 size_t analyse_scratch_bytes(int tdms, int nsamp, int bin_pow2) {
     return scratch_bytes_for((long long)tdms * (nsamp >> bin_pow2));
 }
@@ -445,7 +449,7 @@ extern "C" int pv_analyse_noalloc(const float* d_data, long long ld, int tdms, i
     void* scratch = nullptr;
     PV_TRY(noalloc_scratch(&scratch));
     // Nothing in the scratch needs clearing: every count, offset and the total are written before they
-    // are read, and the counter is 0 between calls.
+    // are read, and each call leaves the counter at 0.
     long long* d_total = reinterpret_cast<long long*>(static_cast<char*>(scratch) + kNoAllocScratch);
     cudaStream_t s = pv::as_stream(stream);
     PV_TRY(pv::analyse_launch(d_data, ld, tdms, nsamp, threshold, rms, bin_pow2, d_events, cap,

@@ -765,7 +765,7 @@ int run_channelise(pv_ppf* h, const void* d_in, int in_int16, int nsub, int npol
         return PV_ERR_ARG;
     }
     // complex spectra of two polarisations: the two-phase kernel as well
-    const bool spectra = mode == 0 && npol == 2 && !in_int16 && h->ntaps == kFastTaps && nblocks >= kFastTaps - 1 &&
+    const bool spectra = mode == 0 && npol == 2 && nsub <= 65535 && !in_int16 && h->ntaps == kFastTaps && nblocks >= kFastTaps - 1 &&
                          (h->nchan == 16 || h->nchan == 32) && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0 &&
                          (reinterpret_cast<uintptr_t>(d_spectra) & 15) == 0;
     if ((fast || spectra) && (pkt_bytes > 0 || getenv("PV_CHAN_GENERIC") == nullptr)) {

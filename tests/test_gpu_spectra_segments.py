@@ -64,3 +64,13 @@ def test_integrator(pv, oracle, cuda, shape, window):
     flat = torch.zeros(d.numel() + 1, device=cuda)
     flat[1:] = d.reshape(-1)
     assert np.array_equal(pv.integrate(flat[1:].view(shape), window).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("nchan", [16, 64])
+def test_more_subbands_than_a_grid_holds_are_refused(pv, cuda, nchan):
+    """The limit of complex spectra is one of the entry point, not of a kernel."""
+    import torch
+    x = torch.zeros(65536, 2, 7 * nchan, dtype=torch.complex64, device=cuda)
+    with pytest.raises(pv.PvError, match="too many subbands"):
+        pv.PPF(nchan, 8).run(x)
+    assert pv.PPF(nchan, 8).run(x[:65535]).shape[1] == 65535

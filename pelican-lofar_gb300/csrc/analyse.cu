@@ -368,16 +368,17 @@ extern "C" int pv_analyse(const float* d_data, long long ld, int tdms, int nsamp
     }
     cudaStream_t s = pv::as_stream(stream);
     pv::Scratch scratch;
-    PV_TRY(pv::scratch_take(&scratch, pv::analyse_scratch_bytes(tdms, nsamp, bin_pow2)));
+    PV_TRY(pv::scratch_take(&scratch, pv::analyse_scratch_bytes(tdms, nsamp, bin_pow2), s));
     // the total goes straight to host memory
-    int rc = pv::analyse_launch(d_data, ld, tdms, nsamp, threshold, rms, bin_pow2, d_events, cap, scratch.host,
+    long long* total = static_cast<long long*>(scratch.host);
+    int rc = pv::analyse_launch(d_data, ld, tdms, nsamp, threshold, rms, bin_pow2, d_events, cap, total,
                                 scratch.dev, s);
     if (rc == PV_OK) rc = pv::cuda_status(cudaStreamSynchronize(s), "synchronise");
     if (rc != PV_OK) {  // its kernels may not have run to their end
         pv::scratch_drop(scratch);
         return rc;
     }
-    *h_count = *static_cast<volatile long long*>(scratch.host);
+    *h_count = *static_cast<volatile long long*>(total);
     pv::scratch_give(scratch);
     return PV_OK;
 }

@@ -18,6 +18,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstdlib>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <type_traits>
@@ -1824,31 +1825,6 @@ extern "C" int pv_delay_table(int* d_shifts, const float* d_dmshift, int nchan, 
     return pv::check_launch("delay_table_kernel");
 }
 
-namespace {
-
-// A thread's page-locked staging (reads from it need no copy by the driver).
-struct Staging {
-    void* p = nullptr;
-    size_t bytes = 0;
-    ~Staging() {
-        if (p) cudaFreeHost(p);
-    }
-    int get(size_t n, void** out) {
-        if (bytes < n) {
-            if (p) cudaFreeHost(p);
-            p = nullptr;
-            bytes = 0;
-            PV_CUDA(cudaHostAlloc(&p, n, cudaHostAllocPortable), "allocate staging");
-            bytes = n;
-        }
-        *out = p;
-        return PV_OK;
-    }
-};
-thread_local Staging t_staging;
-
-}  // namespace
-
 extern "C" int pv_dedisperse_ex(float* d_out, long long out_stride, const float* d_in,
                                 long long row_stride, long long row_len, int nchans, int nout,
                                 int tdms, const float* d_dmshift, float start_over_tsamp,
@@ -1861,12 +1837,25 @@ extern "C" int pv_dedisperse_ex(float* d_out, long long out_stride, const float*
     if (tdms == 0 || nout == 0) return PV_OK;
     std::vector<float> h(nchans);
     cudaStream_t s = pv::as_stream(stream);
-    void* staging = nullptr;
-    PV_TRY(t_staging.get(sizeof(float) * nchans, &staging));
-    PV_CUDA(cudaMemcpyAsync(staging, d_dmshift, sizeof(float) * nchans, cudaMemcpyDeviceToHost, s),
-            "copy dmshift");
-    PV_CUDA(cudaStreamSynchronize(s), "synchronise");
-    std::copy(static_cast<float*>(staging), static_cast<float*>(staging) + nchans, h.begin());
+    // through page-locked memory where it fits: the driver then copies straight into it
+    const size_t bytes = sizeof(float) * nchans;
+    pv::Scratch staging;
+    if (bytes <= pv::kScratchHost && pv::scratch_take(&staging, 0, s) != PV_OK) {
+        cudaGetLastError();  // the call can do without
+        staging = pv::Scratch{};
+    }
+    cudaError_t e = cudaMemcpyAsync(staging.host ? staging.host : h.data(), d_dmshift, bytes,
+                                    cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (staging.host) {
+        if (e == cudaSuccess) {
+            std::memcpy(h.data(), staging.host, bytes);
+            pv::scratch_give(staging);
+        } else {
+            pv::scratch_drop(staging);
+        }
+    }
+    PV_CUDA(e, "copy dmshift");
     // Every delay must be a finite, non-negative sample count: the tiles
     // address shared memory and the input relative to the first trial's delay.
     if (!(start_over_tsamp >= 0.0f) || !(step_over_tsamp >= 0.0f) ||

@@ -76,14 +76,16 @@ cudaError_t allow_max_dynamic_smem(Kernel kern, size_t* limit = nullptr) {
 }
 
 // Scratch of a call that waits for its work before it returns: device memory
-// (cleared when it was allocated) and 64 bytes of host memory that kernels can
-// write.  scratch_give wants it idle; scratch_drop frees it.
+// (cleared on s when it is allocated) and kScratchHost bytes of page-locked
+// host memory that kernels can write.  scratch_give wants it idle;
+// scratch_drop frees it.
+constexpr size_t kScratchHost = 65536;
 struct Scratch {
     void* dev = nullptr;
-    long long* host = nullptr;
+    void* host = nullptr;
     size_t bytes = 0;
 };
-int scratch_take(Scratch* out, size_t bytes);
+int scratch_take(Scratch* out, size_t bytes, cudaStream_t s);
 void scratch_give(const Scratch& b);
 void scratch_drop(const Scratch& b);
 

@@ -19,7 +19,7 @@ std::vector<int> g_sm_counts;
 // result gives its block back idle, so the next one takes it as it is;
 // cudaMallocAsync and cudaFreeAsync around the same call cost 0.2 ms where
 // another copy on the stream followed (the analyser's event list).
-constexpr size_t kScratchKeep = 8, kScratchBytes = 16u << 20;
+constexpr size_t kScratchKeep = 32, kScratchBytes = 16u << 20;
 std::mutex g_scratch_mutex;
 struct Kept {
     int device;
@@ -63,7 +63,7 @@ int smem_optin() {
     return n;
 }
 
-int scratch_take(Scratch* out, size_t bytes) {
+int scratch_take(Scratch* out, size_t bytes, cudaStream_t s) {
     int dev = 0;
     PV_CUDA(cudaGetDevice(&dev), "cudaGetDevice");
     {
@@ -78,9 +78,8 @@ int scratch_take(Scratch* out, size_t bytes) {
     Scratch b;
     b.bytes = bytes < 65536 ? 65536 : bytes;
     cudaError_t e = cudaMalloc(&b.dev, b.bytes);
-    if (e == cudaSuccess) e = cudaMemset(b.dev, 0, b.bytes);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);  // the caller's stream may not wait for it
-    if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&b.host), 64, cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostAlloc(&b.host, kScratchHost, cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaMemsetAsync(b.dev, 0, b.bytes, s);
     if (e != cudaSuccess) {
         set_error("scratch allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
         scratch_drop(b);

@@ -129,6 +129,12 @@ int pv_dedisp_plan_create(pv_dedisp_plan** plan, const float* h_dmshift, int nch
 void pv_dedisp_plan_destroy(pv_dedisp_plan* plan);
 /* Largest integer delay of the plan (samples). */
 int pv_dedisp_plan_max_shift(const pv_dedisp_plan* plan);
+/* The tile that pv_dedisp_plan_run takes on this device for nout samples of
+ * linear rows (ring_len 0) or of a ring, from a 16-byte aligned base and, for
+ * a ring, rows of whole 16 bytes: trials, samples and channels per pipeline
+ * stage; all 0 where a plain kernel runs instead of the pipeline. */
+int pv_dedisp_plan_tile(const pv_dedisp_plan* plan, int nout, long long ring_len, int* trials, int* samples,
+                        int* channels);
 /* PV_OK, or PV_ERR_TIMEOUT if a pipelined launch's bounded wait gave up
  * (synchronous read of the plan's device status word). */
 int pv_dedisp_plan_status(const pv_dedisp_plan* plan, int* h_status);

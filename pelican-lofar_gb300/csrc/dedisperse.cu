@@ -370,7 +370,9 @@ __device__ __forceinline__ void tma_producer(const DedispArgs& a, const Pipe<CS,
 
 // Linear rows without the pipeline: one warp writes samples [t, end) of trial
 // d, the same sums read from global memory.  For a consumer whose wait gave
-// up, so that no call on linear rows can fail after its launch.
+// up, so that no call on linear rows can fail after its launch.  In line: a
+// call by reference makes the kernel's parameters addressable, and its loop 10
+// to 40 % slower.
 __device__ __forceinline__ void direct_sums(const DedispArgs& a, int d, long long t, long long end) {
     const int lane = threadIdx.x & 31;
     const float dv = pv_trial_value(d, a.start, a.step);
@@ -1265,6 +1267,22 @@ constexpr TmaTile kTmaTiles[] = {{16, 1024, 8, 2, 1.0f, 0.0f, 0},  {16, 1024, 2,
                                  {8, 1024, 8, 2, 0.95f, 0.0f, 0},  {8, 256, 16, 2, 0.93f, 0.0f, 0},
                                  {14, 1056, 8, 2, 1.27f, 0.02f, 2}, {8, 1056, 8, 2, 1.28f, 0.03f, 3}};
 constexpr int kOneTrialTiles = 4, kTiles = 6;
+// What a tile spends beside its channels.  Its stores, in channels: the
+// intercepts of times over 1 to 256 channels of 1024 trials x 16384 samples,
+// 23 us + 1.9 us a channel for one trial per warp, 82 us + 1.16 us for pairs (a
+// lane's 33 samples are adjacent, so its stores are 132 bytes from its
+// neighbour's).  And for each round of the CTAs that an SM holds 3.5 us
+// (barriers, the first copies' latency), in adds at the first tile's rate and
+// in cycles: 16 trials x 100000 samples, one round of 16 x 1024 5.5 us + 0.285
+// us a channel, two rounds of 8 x 256 11.5 us + 0.21 us.
+// The tiles' rates were measured on 496 channels and more and hold these
+// already, so they count in full for few channels and not from 512 on.
+inline double few_channels(int nchan) { return std::max(0.0, 1.0 - nchan / 512.0); }
+constexpr double kOneTrialStores = 5.0, kPairStores = 64.0, kRoundAdds = 200e3, kRoundCycles = 5000.0;
+// Up to here the plain kernel, which has no pipeline to fill: 1024 trials x
+// 16384 samples x 4 channels 25 us, one trial per warp 29, pairs 85; at 8
+// channels 39, 37 and 88.
+constexpr int kPlainChannels = 4;
 // Narrow tiles of the one-trial kernel, for calls of few trials or samples and
 // for delays that differ by hundreds of samples from one trial to the next
 // (whose wide tiles do not fit shared memory): trials x parts x samples a
@@ -1285,45 +1303,58 @@ struct NarrowTile {
 constexpr NarrowTile kNarrowTiles[] = {{8, 1, 8, 32, 2}, {4, 1, 8, 32, 2}, {4, 4, 8, 8, 2},
                                        {2, 4, 8, 8, 2},  {1, 4, 8, 8, 3},  {1, 2, 4, 32, 2}};
 
-// SM cycles per channel of the busiest SM: rounds of the resident CTAs, each
+// SM cycles per channel (of nchan) of the busiest SM: rounds of the resident CTAs, each
 // stage at the larger of its shared-memory reads, its copies through L2 and a
 // stage's latency over the stages in flight.  The constants are a fit to 340
 // launches of 25 tiles on 37 shapes (one standard deviation 20 %).
-inline double pipe_cycles(const NarrowTile& t, int sp, int tdms, int nout) {
+inline double pipe_cycles(const NarrowTile& t, int sp, int nchan, int tdms, int nout, int sms) {
     const double copied = 4.0 * (t.tt() + 0.5 * sp) / 38.0;
     const size_t smem = tma_smem(t.st, t.cs, (t.tt() + sp + 8 + 3) & ~3) + 1024;
     const int threads = 32 * (t.dms * t.parts + 1);
     const long long held = std::max(1LL, std::min({(long long)(227 * 1024 / smem), 65536LL / (threads * (40 + t.r)),
                                                    2048LL / threads}));
-    const long long ctas = ceil_div((long long)ceil_div(tdms, t.dms) * ceil_div(nout, t.tt()), (long long)sm_count());
+    const long long ctas = ceil_div((long long)ceil_div(tdms, t.dms) * ceil_div(nout, t.tt()), (long long)sms);
     const auto round = [&](long long q) {
         return std::max({q * t.dms * t.parts * (t.r + 2) / 0.95, q * copied,
                          (2250.0 / t.cs + 6.9 * (t.r + 3.8) + copied) / t.st});
     };
-    return ctas / held * round(held) + (ctas % held ? round(ctas % held) : 0.0);
+    return ctas / held * round(held) + (ctas % held ? round(ctas % held) : 0.0) +
+           few_channels(nchan) * (double)ceil_div(ctas, held) * kRoundCycles / nchan;
 }
 
-// The tile with the least expected time, -1 if none fits: the busiest SM's
-// share of the adds, at a rate that falls where a tile copies more than 0.55
+// The tile with the least expected time, -1 (the plain kernels) for few
+// channels or if none fits: the busiest SM's share of the adds, at a rate that falls where a tile copies more than 0.55
 // bytes per add through L2.  Delays differ most in the lowest channel: half
 // that difference, a seventh of the spread of eight trials, stands for a
 // pair's mean one (measured: 0.4 to 0.5 of it).  A last round that does not
 // fill the SM's residency runs at the 0.6th power of the part it fills
 // (measured for 1 of 2 and 2 of 3 CTAs: 0.65 and 0.74).
 template <typename F>
-int tma_tile(int tdms, int nout, long long ring_len, F spread) {
+int tma_tile(int nchan, int tdms, int nout, long long ring_len, F spread) {
+    if (nchan <= kPlainChannels) return -1;
+    const int sms = sm_count();
+    const double few = few_channels(nchan);
     const auto smem_of = [](const TmaTile& t, int sp) { return tma_smem(t.st, t.cs, (t.tt + sp + 8 + 3) & ~3); };
     // two stages fit, every copy (span + 16-byte rounding) in one ring turn, and the tiles in a grid
     const auto fits = [&](const TmaTile& t, int sp) {
         return smem_of(t, sp) <= 220 * 1024 && ceil_div(tdms, t.dms) <= 65535 &&
                (ring_len <= 0 || ring_len >= (long long)std::min(t.tt, nout) + sp + 8);
     };
+    const auto busiest_of = [&](const TmaTile& t) {
+        return std::ceil((double)ceil_div(tdms, t.dms) * ceil_div(nout, t.tt) / sms);
+    };
+    const auto held_of = [&](const TmaTile& t, int sp) {
+        const int by_smem = (int)(227 * 1024 / (smem_of(t, sp) + 1024));
+        return std::min(by_smem, t.resident ? t.resident : 65536 / (32 * (t.dms + 1) * (t.dms == 8 && t.tt == 1024 ? 80 : 56)));
+    };
     const auto time_of = [&](const TmaTile& t, int sp, double rate, double busiest) {
         const double copied = 4.0 * (t.tt + sp) / ((double)t.tt * t.dms);
-        return busiest * t.dms * t.tt / rate * std::max(1.0, copied / 0.55);
-    };
-    const auto busiest_of = [&](const TmaTile& t) {
-        return std::ceil((double)ceil_div(tdms, t.dms) * ceil_div(nout, t.tt) / sm_count());
+        const double adds = busiest * t.dms * t.tt / rate;
+        double time = adds * nchan * std::max(1.0, copied / 0.55);
+        if (few > 0.0)
+            time += few * (adds * (t.resident ? kPairStores : kOneTrialStores) +
+                           std::ceil(busiest_of(t) / std::max(1, held_of(t, sp))) * kRoundAdds);
+        return time;
     };
     int best = -1;
     double best_t = 0.0;
@@ -1344,7 +1375,7 @@ int tma_tile(int tdms, int nout, long long ring_len, F spread) {
         const double rate = t.rate - t.slope * 0.5 * diff;
         const int sp = guess(t.dms);  // exact only where it could win: the host pays for each spread
         if (rate <= 0.5) continue;
-        const double held = std::min(t.resident, (int)(227 * 1024 / (smem_of(t, sp) + 1024)));
+        const double held = held_of(t, sp);
         if (held < 1.0) continue;
         double busiest = busiest_of(t);
         const double part = std::fmod(busiest, held) / held;
@@ -1360,12 +1391,12 @@ int tma_tile(int tdms, int nout, long long ring_len, F spread) {
     double now = 1e30;
     if (best >= 0) {
         const TmaTile& t = kTmaTiles[best];
-        now = 0.93 * pipe_cycles({t.dms, 1, t.tt / 32, t.cs, t.st}, spread(t.dms), tdms, nout);
+        now = 0.93 * pipe_cycles({t.dms, 1, t.tt / 32, t.cs, t.st}, spread(t.dms), nchan, tdms, nout, sms);
     }
     for (int v = 0; v < (int)(sizeof(kNarrowTiles) / sizeof(kNarrowTiles[0])); ++v) {
         const NarrowTile& t = kNarrowTiles[v];
         if (ceil_div(tdms, t.dms) > 65535) continue;
-        const double cycles = pipe_cycles(t, guess(t.dms), tdms, nout);
+        const double cycles = pipe_cycles(t, guess(t.dms), nchan, tdms, nout, sms);
         if (cycles >= now) continue;
         const int sp = t.dms == 1 ? 0 : spread(t.dms);
         if (tma_smem(t.st, t.cs, (t.tt() + sp + 8 + 3) & ~3) > 220 * 1024 ||
@@ -1377,9 +1408,30 @@ int tma_tile(int tdms, int nout, long long ring_len, F spread) {
     return best;
 }
 
-// Chooses the tile for the delay spread: the widest trial tile whose channel
-// slots fit in shared memory with two buffers of CS channels.  spread(dms) is
-// the largest delay spread of dms trials (delay_spread).
+// The pipeline's tile for rows that bulk copies can fetch (linear rows, or
+// rings of whole 16 bytes, from an aligned base), or -1 for the plain kernels:
+// of these the widest trial tile whose two buffers fit shared memory.
+// spread(dms) is the largest delay spread of dms trials (delay_spread).
+template <typename F>
+struct PlainTiles {
+    F spread;
+    bool fits16() const { return (size_t)2 * 4 * (1024 + spread(16)) * 4 <= 200 * 1024; }
+    bool fits8() const { return (size_t)2 * 4 * (1024 + spread(8)) * 4 <= 220 * 1024; }
+    bool fits4() const { return (size_t)2 * 2 * (512 + spread(4)) * 4 <= 220 * 1024; }
+};
+template <typename F>
+int pipeline_tile(int nchan, int tdms, int nout, long long ring_len, F spread) {
+    const PlainTiles<F> plain{spread};
+    // A ring that the plain kernels refuse (shorter than their tile's span) stays refused where a
+    // narrower tile's span would fit.
+    if (ring_len > 0) {
+        const int tt = plain.fits16() || plain.fits8() ? 1024 : 512;
+        const int dms = plain.fits16() ? 16 : plain.fits8() ? 8 : plain.fits4() ? 4 : 1;
+        if (ring_len < (long long)std::min(tt, nout) + spread(dms)) return -1;
+    }
+    return tma_tile(nchan, tdms, nout, ring_len, spread);
+}
+
 template <typename F>
 int dedisperse_device(float* out, long long out_stride, const float* in, long long row_stride,
                       long long row_len, long long ring_len, long long t_base, int nchan, int nout,
@@ -1391,22 +1443,12 @@ int dedisperse_device(float* out, long long out_stride, const float* in, long lo
     }
     DedispArgs a{out, out_stride, in, row_stride, row_len, ring_len, t_base % std::max(ring_len, 1LL),
                  d_dmshift, nchan, nout, tdms, start, step, 0, wait_ns(), 0};
-    // the plain kernels: the widest trial tile whose two buffers fit shared memory
-    const auto fits16 = [&] { return (size_t)2 * 4 * (1024 + spread(16)) * 4 <= 200 * 1024; };
-    const auto fits8 = [&] { return (size_t)2 * 4 * (1024 + spread(8)) * 4 <= 220 * 1024; };
-    const auto fits4 = [&] { return (size_t)2 * 2 * (512 + spread(4)) * 4 <= 220 * 1024; };
     // Rows whose 16-byte units bulk copies can fetch go through the pipeline.
     const bool aligned = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
     const bool ring = ring_len > 0 && ring_len % 4 == 0 && row_stride % 4 == 0;
     if (ring_len == 0) status = nullptr;  // direct_sums: nothing to report
     if (aligned && (ring ? status != nullptr : ring_len == 0) && getenv("PV_DEDISP_V1") == nullptr) {
-        // A ring that the plain kernels refuse (shorter than their tile's span) stays refused where a
-        // narrower tile's span would fit.
-        const bool plain_ok = ring_len == 0 || [&] {
-            const int tt = fits16() || fits8() ? 1024 : 512, dms = fits16() ? 16 : fits8() ? 8 : fits4() ? 4 : 1;
-            return ring_len >= (long long)std::min(tt, nout) + spread(dms);
-        }();
-        const int v = plain_ok ? tma_tile(tdms, nout, ring_len, spread) : -1;
+        const int v = pipeline_tile(nchan, tdms, nout, ring_len, spread);
         if (v >= 0) {
             a.stall = take_stall();
             const int sp = spread(v < kTiles ? kTmaTiles[v].dms : kNarrowTiles[v - kTiles].dms);
@@ -1424,9 +1466,10 @@ int dedisperse_device(float* out, long long out_stride, const float* in, long lo
             return launch_dedisperse_tma<1, 2, 4, 32, 2>(a, sp, status, s);
         }
     }
-    if (fits16()) return launch_dedisperse<16, 32, 4>(a, spread(16), s);
-    if (fits8()) return launch_dedisperse<8, 32, 4>(a, spread(8), s);
-    if (fits4()) return launch_dedisperse<4, 16, 2>(a, spread(4), s);
+    const PlainTiles<F> plain{spread};
+    if (plain.fits16()) return launch_dedisperse<16, 32, 4>(a, spread(16), s);
+    if (plain.fits8()) return launch_dedisperse<8, 32, 4>(a, spread(8), s);
+    if (plain.fits4()) return launch_dedisperse<4, 16, 2>(a, spread(4), s);
     return launch_dedisperse<1, 16, 1>(a, spread(1), s);
 }
 
@@ -2001,6 +2044,27 @@ extern "C" int pv_dedisp_plan_clear_status(pv_dedisp_plan* p, void* stream) {
 }
 
 extern "C" int pv_dedisp_plan_max_shift(const pv_dedisp_plan* p) { return p ? p->max_shift : -1; }
+
+extern "C" int pv_dedisp_plan_tile(const pv_dedisp_plan* p, int nout, long long ring_len, int* trials, int* samples,
+                                   int* channels) {
+    if (!p || nout <= 0 || ring_len < 0 || !trials || !samples || !channels) {
+        pv::set_error("pv_dedisp_plan_tile: invalid arguments");
+        return PV_ERR_ARG;
+    }
+    const int v = ring_len % 4 ? -1
+                               : pv::pipeline_tile(p->nchan, p->tdms, nout, ring_len,
+                                                   [p](int dms) { return p->spread(dms); });
+    if (v < 0) {
+        *trials = *samples = *channels = 0;
+    } else if (v < pv::kTiles) {
+        const pv::TmaTile& t = pv::kTmaTiles[v];
+        *trials = t.dms, *samples = t.tt, *channels = t.cs;
+    } else {
+        const pv::NarrowTile& t = pv::kNarrowTiles[v - pv::kTiles];
+        *trials = t.dms, *samples = t.tt(), *channels = t.cs;
+    }
+    return PV_OK;
+}
 
 extern "C" int pv_dedisp_plan_run(const pv_dedisp_plan* p, float* d_out, long long out_stride,
                                   const float* d_in, long long row_stride, long long row_len,

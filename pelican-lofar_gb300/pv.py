@@ -132,6 +132,7 @@ def _declare(L):
         "pv_ddmod_add": (i, [vp, vp, i, i, i, i, d, P(i), vp]),
         "pv_ddmod_pop": (i, [vp, vp, ll, P(i), P(ll), vp]),
         "pv_ddmod_params": (i, [vp, P(i)]),
+        "pv_dedisp_plan_tile": (i, [vp, i, ll, P(i), P(i), P(i)]),
         "pv_dedisp_plan_status": (i, [vp, P(i)]),
         "pv_dedisp_plan_clear_status": (i, [vp, vp]),
         "pv_set_wait_limit": (ll, [ll]),
@@ -234,6 +235,13 @@ class DedispPlan:
 
     def max_shift(self):
         return load().pv_dedisp_plan_max_shift(self.h)
+
+    def tile(self, nout, ring_len=0):
+        """(trials, samples, channels per stage) of the tile that run takes; zeros: a plain kernel."""
+        t = (C.c_int * 3)()
+        at = [C.cast(C.addressof(t) + 4 * k, C.POINTER(C.c_int)) for k in range(3)]
+        check(load().pv_dedisp_plan_tile(self.h, nout, ring_len, *at))
+        return tuple(t)
 
     def run(self, d_in, nout, out=None, ring_len=0, t_base=0, row_len=None, stream=None):
         """d_in: float32 [nchan][row_stride] -> out [tdms][nout] (ring rows

@@ -156,3 +156,49 @@ def test_short_ring_stays_refused(pv, cuda):
     x = torch.zeros(33, 1600, device=cuda)
     with pytest.raises(Exception):
         plan.run(x, 1000, ring_len=1600)
+
+
+TILES = [
+    # (trials, samples, channels per stage) of each tile on 152 SMs, zeros for the plain kernel; one
+    # trial and one sample more than whole tiles
+    ((0, 0, 0), (4, 1009, 9001, 150.0, -0.05, 30.0)),
+    ((16, 1024, 8), (24, 513, 10241, 150.0, -0.05, 100.0)),
+    ((16, 1024, 2), (90, 65, 20481, 150.0, -0.1, 10000.0)),
+    ((8, 1024, 8), (33, 161, 18433, 150.0, -0.05, 3089.0)),
+    ((8, 256, 16), (70, 297, 5121, 150.0, -0.05, 300.0)),
+    ((14, 1056, 8), (200, 169, 21121, 150.0, -0.05, 763.0)),
+    ((8, 1056, 8), (300, 257, 10561, 150.0, -0.1, 4.0)),
+    ((8, 256, 32), (128, 153, 3329, 150.0, -0.05, 4745.0)),
+    ((4, 256, 32), (65, 101, 3073, 150.0, -0.05, 5.0)),
+    ((4, 1024, 8), (200, 73, 15361, 150.0, -0.05, 54.0)),
+    ((2, 1024, 8), (90, 39, 11265, 150.0, -0.05, 18853.0)),
+    ((1, 1024, 8), (70, 8, 29697, 150.0, -0.1, 21752.0)),
+    ((1, 256, 32), (70, 7, 3585, 150.0, -0.1, 166.0)),
+]
+
+
+@pytest.mark.parametrize("ring", [False, True])
+@pytest.mark.parametrize("tile,case", TILES)
+def test_every_tile(pv, oracle, cuda, tile, case, ring):
+    """Each tile on sizes that the rule gives it, so that a change of the rule
+    cannot leave one untested."""
+    import torch
+    if torch.cuda.get_device_properties(0).multi_processor_count != 152:
+        pytest.skip("the tiles of 152 SMs")
+    k, start, step, ms, _ = _case(pv, oracle, case)
+    plan = pv.DedispPlan(k, case[1], float(start), float(step))
+    assert plan.tile(case[2], (case[2] + ms + 1100 + 3) // 4 * 4 if ring else 0) == tile
+    test_trial_pairs(pv, oracle, cuda, case, ring)
+
+
+@pytest.mark.parametrize("nchan", [1, 2, 4, 5, 8, 32])
+def test_few_channels_take_no_trial_pairs(pv, oracle, cuda, nchan):
+    """A pair's stores cost what 64 channels do (1024 trials x 16384 samples of
+    one channel: 83 us against 17 by the plain kernel)."""
+    import torch
+    if torch.cuda.get_device_properties(0).multi_processor_count != 152:
+        pytest.skip("the tiles of 152 SMs")
+    k, _ = pv.dm_shifts(150.0, -0.05, nchan)
+    plan = pv.DedispPlan(k, 1024, 0.0, 1.0)
+    for ring in (0, 18000):
+        assert plan.tile(16384, ring) == ((0, 0, 0) if nchan <= 4 else (16, 1024, 8))

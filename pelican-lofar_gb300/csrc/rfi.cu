@@ -882,64 +882,20 @@ __global__ void __launch_bounds__(P, P == 256 ? 6 : (P == 512 ? 3 : 1)) rfi_appl
                           J.flags ? J.flags + (long long)(t0 + i) * J.cfg.nbins : nullptr, i, i == n - 1);
 }
 
-template <int P, int KM, bool PLAIN>
-int rfi_blocks_t(const RfiJob* jobs, const RfiJob& one, int njobs, const pv::BeamStep* bs, int nt, cudaStream_t s) {
-    for (int t0 = 0; t0 < nt; t0 += kRfiBlock) {
-        const int n = std::min(kRfiBlock, nt - t0);
-        for (int second = 0; second < 2; ++second) {
-            rfi_stats_kernel<P, KM, PLAIN><<<dim3((unsigned)n, (unsigned)njobs), P, 0, s>>>(jobs, one, bs, t0, second);
-            PV_TRY(pv::check_launch("rfi_stats_kernel"));
-            rfi_scan_kernel<P><<<(unsigned)njobs, kScanThreads, 0, s>>>(jobs, one, bs, t0, n, second);
-            PV_TRY(pv::check_launch("rfi_scan_kernel"));
-        }
-        rfi_apply_kernel<P, KM, PLAIN><<<dim3((unsigned)n + 1, (unsigned)njobs), P, 0, s>>>(jobs, one, bs, t0, n);
-        PV_TRY(pv::check_launch("rfi_apply_kernel"));
-    }
-    return PV_OK;
-}
-
-// Channel counts that share the launches of rfi_blocks: the largest one of
-// the class (0x7fffffff: any number of channels per thread).
-int rfi_blocks_class(int nbins) {
-    for (int top : {1024, 4096, 8192, 16384})
-        if (nbins <= top) return top;
-    return 0x7fffffff;
-}
-// One polarisation and a flat bandpass: kernels without the general addressing
-// and bandpass, whose registers let a third more CTAs share an SM.
-bool rfi_plain(const RfiConfig& cfg, const RfiBuffers& bufs, int npol) {
-    return npol == 1 && cfg.deg == 0 && bufs.killed == nullptr;
-}
-
-// nt spectra of one beam (jobs null), or of the njobs beams of one class of a
-// batch; nbins is their largest channel count (or the class).
-template <bool PLAIN>
-int rfi_blocks_p(int nbins, const RfiJob* jobs, const RfiJob& one, int njobs, const pv::BeamStep* bs, int nt,
-                 cudaStream_t s) {
-    if (nbins <= 1024) return rfi_blocks_t<256, 4, PLAIN>(jobs, one, njobs, bs, nt, s);
-    if (nbins <= 4096) return rfi_blocks_t<512, 8, PLAIN>(jobs, one, njobs, bs, nt, s);
-    if (nbins <= 8192) return rfi_blocks_t<1024, 8, PLAIN>(jobs, one, njobs, bs, nt, s);
-    if (nbins <= 16384) return rfi_blocks_t<1024, 16, PLAIN>(jobs, one, njobs, bs, nt, s);
-    return rfi_blocks_t<1024, 0, PLAIN>(jobs, one, njobs, bs, nt, s);
-}
-int rfi_blocks(int nbins, bool plain, const RfiJob* jobs, const RfiJob& one, int njobs, const pv::BeamStep* bs, int nt,
-               cudaStream_t s) {
-    return plain ? rfi_blocks_p<true>(nbins, jobs, one, njobs, bs, nt, s)
-                 : rfi_blocks_p<false>(nbins, jobs, one, njobs, bs, nt, s);
-}
-
 // The clippers of many beams at once: cluster b (CTAs b*C .. b*C+C-1) runs
-// job b (every job of a launch has the same partial count); beams without a
-// chunk this step return at once.
+// spectra [t0, t0 + n) of job b (every job of a launch has the same partial
+// count); beams without a chunk this step return at once.
 template <int T, int C>
 __global__ void __launch_bounds__(T, 1) rfi_batch_kernel(const RfiJob* __restrict__ jobs,
-                                                         const pv::BeamStep* __restrict__ bs) {
+                                                         const pv::BeamStep* __restrict__ bs, int t0, int n) {
     const int job = blockIdx.x / C;
     if (bs && !bs[jobs[job].beam].active) return;  // the whole cluster returns
     const RfiConfig cfg = jobs[job].cfg;
     const RfiBuffers bufs = jobs[job].bufs;
     const Geo geo = jobs[job].geo;
-    rfi_body<T, C>(cfg, bufs, jobs[job].data, jobs[job].nt, geo, jobs[job].flags, (int)(blockIdx.x % C));
+    float* data = jobs[job].data + (long long)t0 * geo.nsub * geo.npol * geo.nchan;
+    unsigned char* flags = jobs[job].flags ? jobs[job].flags + (long long)t0 * cfg.nbins : nullptr;
+    rfi_body<T, C>(cfg, bufs, data, n, geo, flags, (int)(blockIdx.x % C));
 }
 
 // Threads per CTA and CTAs per beam for a partial count.  split 0: one CTA
@@ -996,30 +952,33 @@ int rfi_launch_ex(K kern, int clusters, int C, int T, size_t smem, cudaStream_t 
 }
 
 // Sets the shared-memory attribute of both kernels of a shape and launches
-// one of them: jobs != null selects the batched kernel (nblocks jobs;
-// nblocks == 0: the attribute only, before any stream capture).
+// one of them on spectra [t0, t0 + nt): jobs != null selects the batched
+// kernel (nblocks jobs; nblocks == 0: the attribute only, before any stream
+// capture).
 template <int T, int C>
 int rfi_launch_t(size_t smem, int nblocks, const RfiJob* jobs, const pv::BeamStep* bs,
-                 const RfiConfig& cfg, const RfiBuffers& bufs, float* data, int nt, const Geo& geo,
+                 const RfiConfig& cfg, const RfiBuffers& bufs, float* data, int t0, int nt, const Geo& geo,
                  unsigned char* flags, cudaStream_t s) {
     if (jobs) {
         if (nblocks == 0) return rfi_set_smem(rfi_batch_kernel<T, C>, smem);
-        PV_TRY(rfi_launch_ex(rfi_batch_kernel<T, C>, nblocks, C, T, smem, s, jobs, bs));
+        PV_TRY(rfi_launch_ex(rfi_batch_kernel<T, C>, nblocks, C, T, smem, s, jobs, bs, t0, nt));
         return pv::check_launch("rfi_batch_kernel");
     }
     PV_TRY(rfi_set_smem(rfi_kernel<T, C>, smem));
+    data += (long long)t0 * geo.nsub * geo.npol * geo.nchan;
+    if (flags) flags += (long long)t0 * cfg.nbins;
     PV_TRY(rfi_launch_ex(rfi_kernel<T, C>, 1, C, T, smem, s, cfg, bufs, data, nt, geo, flags));
     return pv::check_launch("rfi_kernel");
 }
 
 int rfi_launch(int parts, int split, size_t smem, int nblocks, const RfiJob* jobs, const pv::BeamStep* bs,
-               const RfiConfig& cfg, const RfiBuffers& bufs, float* data, int nt, const Geo& geo,
+               const RfiConfig& cfg, const RfiBuffers& bufs, float* data, int t0, int nt, const Geo& geo,
                unsigned char* flags, cudaStream_t s) {
     int T = 0, C = 0;
     rfi_shape(parts, split, &T, &C);
 #define PV_RFI_SHAPE(TT, CC)                                                                          \
     if (T == TT && C == CC)                                                                          \
-        return rfi_launch_t<TT, CC>(smem, nblocks, jobs, bs, cfg, bufs, data, nt, geo, flags, s);
+        return rfi_launch_t<TT, CC>(smem, nblocks, jobs, bs, cfg, bufs, data, t0, nt, geo, flags, s);
     PV_RFI_SHAPE(256, 1)
     PV_RFI_SHAPE(512, 1)
     PV_RFI_SHAPE(1024, 1)
@@ -1029,6 +988,71 @@ int rfi_launch(int parts, int split, size_t smem, int nblocks, const RfiJob* job
 #undef PV_RFI_SHAPE
     pv::set_error("RFI_Clipper: no kernel for %d partial sums", parts);
     return PV_ERR_ARG;
+}
+
+// Shared memory of a walk by a clipper whose spectra are done in blocks (rfi_shape's split 1).
+size_t rfi_walk_smem(int nbins) {
+    int T = 0, C = 0;
+    rfi_shape(pv_rfi_parts(nbins), 1, &T, &C);
+    return rfi_smem_bytes(nbins, pv_rfi_parts(nbins), T);
+}
+
+// A block of so few spectra is walked: five launches take 60 us, call included,
+// the walk 40 us and 3 to 7 us a spectrum.  us of 2 and 4 spectra, in blocks /
+// walked: 512 channels 61 59 / 45 50, 4096 60 60 / 56 67, with bandpass terms
+// 73 72 / 63 77, 12288 64 63 / 59 73.
+constexpr int rfi_walk_few(int parts) { return parts <= 512 ? 4 : 2; }
+
+template <int P, int KM, bool PLAIN>
+int rfi_blocks_t(const RfiJob* jobs, const RfiJob& one, int njobs, const pv::BeamStep* bs, int nt, size_t walk_smem,
+                 cudaStream_t s) {
+    for (int t0 = 0; t0 < nt; t0 += kRfiBlock) {
+        const int n = std::min(kRfiBlock, nt - t0);
+        if (n <= rfi_walk_few(P)) {
+            PV_TRY(rfi_launch(P, 1, walk_smem, njobs, jobs, bs, one.cfg, one.bufs, one.data, t0, n, one.geo, one.flags,
+                              s));
+            continue;
+        }
+        for (int second = 0; second < 2; ++second) {
+            rfi_stats_kernel<P, KM, PLAIN><<<dim3((unsigned)n, (unsigned)njobs), P, 0, s>>>(jobs, one, bs, t0, second);
+            PV_TRY(pv::check_launch("rfi_stats_kernel"));
+            rfi_scan_kernel<P><<<(unsigned)njobs, kScanThreads, 0, s>>>(jobs, one, bs, t0, n, second);
+            PV_TRY(pv::check_launch("rfi_scan_kernel"));
+        }
+        rfi_apply_kernel<P, KM, PLAIN><<<dim3((unsigned)n + 1, (unsigned)njobs), P, 0, s>>>(jobs, one, bs, t0, n);
+        PV_TRY(pv::check_launch("rfi_apply_kernel"));
+    }
+    return PV_OK;
+}
+
+// Channel counts that share the launches of rfi_blocks: the largest one of
+// the class (0x7fffffff: any number of channels per thread).
+int rfi_blocks_class(int nbins) {
+    for (int top : {1024, 4096, 8192, 16384})
+        if (nbins <= top) return top;
+    return 0x7fffffff;
+}
+// One polarisation and a flat bandpass: kernels without the general addressing
+// and bandpass, whose registers let a third more CTAs share an SM.
+bool rfi_plain(const RfiConfig& cfg, const RfiBuffers& bufs, int npol) {
+    return npol == 1 && cfg.deg == 0 && bufs.killed == nullptr;
+}
+
+// nt spectra of one beam (jobs null), or of the njobs beams of one class of a
+// batch; nbins is their largest channel count (or the class).
+template <bool PLAIN>
+int rfi_blocks_p(int nbins, const RfiJob* jobs, const RfiJob& one, int njobs, const pv::BeamStep* bs, int nt,
+                 size_t walk_smem, cudaStream_t s) {
+    if (nbins <= 1024) return rfi_blocks_t<256, 4, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, s);
+    if (nbins <= 4096) return rfi_blocks_t<512, 8, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, s);
+    if (nbins <= 8192) return rfi_blocks_t<1024, 8, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, s);
+    if (nbins <= 16384) return rfi_blocks_t<1024, 16, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, s);
+    return rfi_blocks_t<1024, 0, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, s);
+}
+int rfi_blocks(int nbins, bool plain, const RfiJob* jobs, const RfiJob& one, int njobs, const pv::BeamStep* bs, int nt,
+               size_t walk_smem, cudaStream_t s) {
+    return plain ? rfi_blocks_p<true>(nbins, jobs, one, njobs, bs, nt, walk_smem, s)
+                 : rfi_blocks_p<false>(nbins, jobs, one, njobs, bs, nt, walk_smem, s);
 }
 
 }  // namespace
@@ -1235,9 +1259,10 @@ extern "C" int pv_rfi_run(pv_rfi* h, float* d_data, int nt, int nsub, int npol, 
     const Geo geo = make_geo(nsub, npol, nchan);
     if (rfi_in_blocks(h) && h->work.rec) {
         const RfiJob one{h->cfg, h->dev, d_data, d_flags, geo, h->work, nt, 0};
-        return rfi_blocks(nbins, rfi_plain(h->cfg, h->dev, npol), nullptr, one, 1, nullptr, nt, s);
+        return rfi_blocks(nbins, rfi_plain(h->cfg, h->dev, npol), nullptr, one, 1, nullptr, nt, rfi_walk_smem(nbins),
+                          s);
     }
-    return rfi_launch(parts, h->split, smem, 1, nullptr, nullptr, h->cfg, h->dev, d_data, nt, geo, d_flags, s);
+    return rfi_launch(parts, h->split, smem, 1, nullptr, nullptr, h->cfg, h->dev, d_data, 0, nt, geo, d_flags, s);
 }
 
 // Back to the state of a clipper that has seen no spectrum (the running
@@ -1435,7 +1460,8 @@ int rfi_batch_create(RfiBatch** out, pv_rfi* const* handles, float* const* data,
             b->classes[k].ctas = C;
             jobs.emplace_back();
         }
-        b->classes[k].smem = std::max(b->classes[k].smem, smem);
+        // a class in blocks walks few spectra as a clipper of its own does
+        b->classes[k].smem = std::max(b->classes[k].smem, blocks ? rfi_walk_smem(nbins) : smem);
         RfiJob j{};
         j.cfg = h->cfg;
         j.bufs = h->dev;
@@ -1473,9 +1499,9 @@ int rfi_batch_create(RfiBatch** out, pv_rfi* const* handles, float* const* data,
                            cudaMemcpyHostToDevice);
         int rc = e == cudaSuccess ? PV_OK : cuda_status(e, "RFI batch jobs");
         // set the kernel attribute now, outside any stream capture
-        if (rc == PV_OK && !c.blocks)
-            rc = rfi_launch(c.parts, b->split, c.smem, 0, c.d_jobs, nullptr, RfiConfig{}, RfiBuffers{}, nullptr, 0,
-                            Geo{}, nullptr, s);
+        if (rc == PV_OK)
+            rc = rfi_launch(c.parts, c.blocks ? 1 : b->split, c.smem, 0, c.d_jobs, nullptr, RfiConfig{}, RfiBuffers{},
+                            nullptr, 0, 0, Geo{}, nullptr, s);
         if (rc != PV_OK) {
             rfi_batch_destroy(b);
             return rc;
@@ -1494,9 +1520,9 @@ int rfi_batch_ctas(const RfiBatch* b, int k) { return b->classes[k].njobs * b->c
 int rfi_batch_launch_one(RfiBatch* b, int k, cudaStream_t s) {
     auto& c = b->classes[k];
     if (c.njobs == 0) return PV_OK;
-    if (c.blocks) return rfi_blocks(c.nbins, c.plain, c.d_jobs, RfiJob{}, c.njobs, b->bs, b->nt, s);
+    if (c.blocks) return rfi_blocks(c.nbins, c.plain, c.d_jobs, RfiJob{}, c.njobs, b->bs, b->nt, c.smem, s);
     return rfi_launch(c.parts, b->split, c.smem, c.njobs, c.d_jobs, b->bs, RfiConfig{}, RfiBuffers{}, nullptr, 0,
-                      Geo{}, nullptr, s);
+                      b->nt, Geo{}, nullptr, s);
 }
 
 }  // namespace pv

@@ -149,3 +149,20 @@ def test_few_and_many_failures_with_full_histories(pv, oracle, cuda, hits, histo
     x *= np.linspace(1.0, 1.05, nt)[:, None]
     bp = make_bp_text(nsub * nchan, START, WIDTH, 1000.0, 50.0)
     _run(pv, oracle, cuda, x.astype(np.float32).reshape(nt, nsub, 1, nchan), (history,), bp, history)
+
+
+@pytest.mark.parametrize("nsub,few", [(8, 4), (65, 4), (320, 2)])
+def test_few_spectra_take_one_launch(pv, oracle, cuda, nsub, few):
+    """Calls of a few spectra, and the few left of a call after its last whole
+    block, are walked: one launch, bit for bit the same."""
+    import torch
+    nt, nchan = 2 * 2048 + few + 1, 16
+    data = stokes_filterbank(np.random.default_rng(nsub), nt, nsub, nchan)
+    bp = make_bp_text(nsub * nchan, START, WIDTH, 1000.0, 50.0)
+    _run(pv, oracle, cuda, data, (1, 1 + few, 1 + few + 2048), bp, 1200)
+    g = pv.RFI(bp, cr=5.0, sr=4.0, history=1200)
+    d = torch.from_numpy(data).to(cuda)
+    for n, want in ((1, 1), (few, 1), (few + 1, 5), (2048 + few, 6)):
+        before = pv.launches()
+        g.run(d[:n])
+        assert pv.launches() - before == want

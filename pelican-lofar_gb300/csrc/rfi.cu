@@ -824,7 +824,14 @@ __device__ __forceinline__ void rfi_body(const RfiConfig& cfg, const RfiBuffers&
 template <int T, int C>
 __global__ void __launch_bounds__(T, 1)
 rfi_kernel(RfiConfig cfg, RfiBuffers bufs, float* __restrict__ data, int nt, Geo geo,
-           unsigned char* __restrict__ flags) {
+           unsigned char* __restrict__ flags, const int* __restrict__ hdr) {
+    if (hdr) {  // what the scan of a block left
+        const int from = hdr[kHdrEnd];
+        if (from >= nt) return;  // the whole cluster
+        data += (long long)from * geo.nsub * geo.npol * geo.nchan;
+        if (flags) flags += (long long)from * cfg.nbins;
+        nt -= from;
+    }
     rfi_body<T, C>(cfg, bufs, data, nt, geo, flags, C > 1 ? (int)cooperative_groups::this_cluster().block_rank() : 0);
 }
 
@@ -858,41 +865,49 @@ template <int P>
 __global__ void __launch_bounds__(kScanThreads, 1) rfi_scan_kernel(const RfiJob* __restrict__ jobs,
                                                                    const __grid_constant__ RfiJob one,
                                                                    const pv::BeamStep* __restrict__ bs, int t0,
-                                                                   int n, bool second) {
+                                                                   int n, bool second, bool may_leave) {
     const RfiJob& J = jobs ? jobs[blockIdx.x] : one;
     if (bs && !bs[J.beam].active) return;
     const long long spec_elems = (long long)J.geo.nsub * J.geo.npol * J.geo.nchan;
-    rfi_scan_body<P>(J.cfg, J.bufs, J.work, J.data + (long long)t0 * spec_elems, J.geo, n, second);
+    rfi_scan_body<P>(J.cfg, J.bufs, J.work, J.data + (long long)t0 * spec_elems, J.geo, n, second, may_leave);
 }
 
 // CTA 0 of a job adds up the fraction of bad channels, CTA 1 + i does spectrum i.
 template <int P, int KM, bool PLAIN>
 __global__ void __launch_bounds__(P, P == 256 ? 6 : (P == 512 ? 3 : 1)) rfi_apply_kernel(const RfiJob* __restrict__ jobs,
                                                       const __grid_constant__ RfiJob one,
-                                                      const pv::BeamStep* __restrict__ bs, int t0, int n) {
+                                                      const pv::BeamStep* __restrict__ bs, int t0) {
     const RfiJob& J = jobs ? jobs[blockIdx.y] : one;
     if (bs && !bs[J.beam].active) return;
     const int i = (int)blockIdx.x - 1;
     if (i < 0) {
-        rfi_fraction<P>(J.cfg, J.bufs, J.work, n);
+        rfi_fraction<P>(J.cfg, J.bufs, J.work);
         return;
     }
     const long long spec_elems = (long long)J.geo.nsub * J.geo.npol * J.geo.nchan;
     rfi_apply_body<P, KM, PLAIN>(J.cfg, J.bufs, J.work, J.data + (long long)(t0 + i) * spec_elems, J.geo,
-                          J.flags ? J.flags + (long long)(t0 + i) * J.cfg.nbins : nullptr, i, i == n - 1);
+                          J.flags ? J.flags + (long long)(t0 + i) * J.cfg.nbins : nullptr, i);
 }
 
 // The clippers of many beams at once: cluster b (CTAs b*C .. b*C+C-1) runs
 // spectra [t0, t0 + n) of job b (every job of a launch has the same partial
-// count); beams without a chunk this step return at once.
+// count), or with rest what the scan of that block left; beams without a chunk
+// this step return at once.
 template <int T, int C>
 __global__ void __launch_bounds__(T, 1) rfi_batch_kernel(const RfiJob* __restrict__ jobs,
-                                                         const pv::BeamStep* __restrict__ bs, int t0, int n) {
+                                                         const pv::BeamStep* __restrict__ bs, int t0, int n,
+                                                         bool rest) {
     const int job = blockIdx.x / C;
     if (bs && !bs[jobs[job].beam].active) return;  // the whole cluster returns
     const RfiConfig cfg = jobs[job].cfg;
     const RfiBuffers bufs = jobs[job].bufs;
     const Geo geo = jobs[job].geo;
+    if (rest) {
+        const int from = jobs[job].work.hdr[kHdrEnd];
+        if (from >= n) return;
+        t0 += from;
+        n -= from;
+    }
     float* data = jobs[job].data + (long long)t0 * geo.nsub * geo.npol * geo.nchan;
     unsigned char* flags = jobs[job].flags ? jobs[job].flags + (long long)t0 * cfg.nbins : nullptr;
     rfi_body<T, C>(cfg, bufs, data, n, geo, flags, (int)(blockIdx.x % C));
@@ -953,32 +968,37 @@ int rfi_launch_ex(K kern, int clusters, int C, int T, size_t smem, cudaStream_t 
 
 // Sets the shared-memory attribute of both kernels of a shape and launches
 // one of them on spectra [t0, t0 + nt): jobs != null selects the batched
-// kernel (nblocks jobs; nblocks == 0: the attribute only, before any stream
-// capture).
+// kernel (nblocks jobs; nblocks == 0: the attributes only, before any stream
+// capture).  rest: only what the scan of these spectra left (hdr: of the one
+// beam).
 template <int T, int C>
 int rfi_launch_t(size_t smem, int nblocks, const RfiJob* jobs, const pv::BeamStep* bs,
                  const RfiConfig& cfg, const RfiBuffers& bufs, float* data, int t0, int nt, const Geo& geo,
-                 unsigned char* flags, cudaStream_t s) {
+                 unsigned char* flags, cudaStream_t s, bool rest, const int* hdr) {
+    if (nblocks == 0) {
+        PV_TRY(rfi_set_smem(rfi_kernel<T, C>, smem));
+        return rfi_set_smem(rfi_batch_kernel<T, C>, smem);
+    }
     if (jobs) {
-        if (nblocks == 0) return rfi_set_smem(rfi_batch_kernel<T, C>, smem);
-        PV_TRY(rfi_launch_ex(rfi_batch_kernel<T, C>, nblocks, C, T, smem, s, jobs, bs, t0, nt));
+        PV_TRY(rfi_launch_ex(rfi_batch_kernel<T, C>, nblocks, C, T, smem, s, jobs, bs, t0, nt, rest));
         return pv::check_launch("rfi_batch_kernel");
     }
-    PV_TRY(rfi_set_smem(rfi_kernel<T, C>, smem));
+    if (!rest) PV_TRY(rfi_set_smem(rfi_kernel<T, C>, smem));  // of a rest: set by setup()
     data += (long long)t0 * geo.nsub * geo.npol * geo.nchan;
     if (flags) flags += (long long)t0 * cfg.nbins;
-    PV_TRY(rfi_launch_ex(rfi_kernel<T, C>, 1, C, T, smem, s, cfg, bufs, data, nt, geo, flags));
+    PV_TRY(rfi_launch_ex(rfi_kernel<T, C>, 1, C, T, smem, s, cfg, bufs, data, nt, geo, flags,
+                         rest ? hdr : nullptr));
     return pv::check_launch("rfi_kernel");
 }
 
 int rfi_launch(int parts, int split, size_t smem, int nblocks, const RfiJob* jobs, const pv::BeamStep* bs,
                const RfiConfig& cfg, const RfiBuffers& bufs, float* data, int t0, int nt, const Geo& geo,
-               unsigned char* flags, cudaStream_t s) {
+               unsigned char* flags, cudaStream_t s, bool rest = false, const int* hdr = nullptr) {
     int T = 0, C = 0;
     rfi_shape(parts, split, &T, &C);
 #define PV_RFI_SHAPE(TT, CC)                                                                          \
     if (T == TT && C == CC)                                                                          \
-        return rfi_launch_t<TT, CC>(smem, nblocks, jobs, bs, cfg, bufs, data, t0, nt, geo, flags, s);
+        return rfi_launch_t<TT, CC>(smem, nblocks, jobs, bs, cfg, bufs, data, t0, nt, geo, flags, s, rest, hdr);
     PV_RFI_SHAPE(256, 1)
     PV_RFI_SHAPE(512, 1)
     PV_RFI_SHAPE(1024, 1)
@@ -1005,7 +1025,7 @@ constexpr int rfi_walk_few(int parts) { return parts <= 512 ? 4 : 2; }
 
 template <int P, int KM, bool PLAIN>
 int rfi_blocks_t(const RfiJob* jobs, const RfiJob& one, int njobs, const pv::BeamStep* bs, int nt, size_t walk_smem,
-                 cudaStream_t s) {
+                 bool may_leave, cudaStream_t s) {
     for (int t0 = 0; t0 < nt; t0 += kRfiBlock) {
         const int n = std::min(kRfiBlock, nt - t0);
         if (n <= rfi_walk_few(P)) {
@@ -1016,11 +1036,15 @@ int rfi_blocks_t(const RfiJob* jobs, const RfiJob& one, int njobs, const pv::Bea
         for (int second = 0; second < 2; ++second) {
             rfi_stats_kernel<P, KM, PLAIN><<<dim3((unsigned)n, (unsigned)njobs), P, 0, s>>>(jobs, one, bs, t0, second);
             PV_TRY(pv::check_launch("rfi_stats_kernel"));
-            rfi_scan_kernel<P><<<(unsigned)njobs, kScanThreads, 0, s>>>(jobs, one, bs, t0, n, second);
+            rfi_scan_kernel<P><<<(unsigned)njobs, kScanThreads, 0, s>>>(jobs, one, bs, t0, n, second,
+                                                                           may_leave);
             PV_TRY(pv::check_launch("rfi_scan_kernel"));
         }
-        rfi_apply_kernel<P, KM, PLAIN><<<dim3((unsigned)n + 1, (unsigned)njobs), P, 0, s>>>(jobs, one, bs, t0, n);
+        rfi_apply_kernel<P, KM, PLAIN><<<dim3((unsigned)n + 1, (unsigned)njobs), P, 0, s>>>(jobs, one, bs, t0);
         PV_TRY(pv::check_launch("rfi_apply_kernel"));
+        if (may_leave)
+            PV_TRY(rfi_launch(P, 1, walk_smem, njobs, jobs, bs, one.cfg, one.bufs, one.data, t0, n, one.geo, one.flags,
+                              s, true, one.work.hdr));
     }
     return PV_OK;
 }
@@ -1034,25 +1058,26 @@ int rfi_blocks_class(int nbins) {
 }
 // One polarisation and a flat bandpass: kernels without the general addressing
 // and bandpass, whose registers let a third more CTAs share an SM.
-bool rfi_plain(const RfiConfig& cfg, const RfiBuffers& bufs, int npol) {
-    return npol == 1 && cfg.deg == 0 && bufs.killed == nullptr;
-}
+bool rfi_flat(const RfiConfig& cfg, const RfiBuffers& bufs) { return cfg.deg == 0 && bufs.killed == nullptr; }
+bool rfi_plain(const RfiConfig& cfg, const RfiBuffers& bufs, int npol) { return npol == 1 && rfi_flat(cfg, bufs); }
 
 // nt spectra of one beam (jobs null), or of the njobs beams of one class of a
-// batch; nbins is their largest channel count (or the class).
+// batch; nbins is their largest channel count (or the class).  may_leave: a
+// scan may leave spectra to the walk, whose launch then follows each block (3
+// to 4 us where it finds nothing left).
 template <bool PLAIN>
 int rfi_blocks_p(int nbins, const RfiJob* jobs, const RfiJob& one, int njobs, const pv::BeamStep* bs, int nt,
-                 size_t walk_smem, cudaStream_t s) {
-    if (nbins <= 1024) return rfi_blocks_t<256, 4, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, s);
-    if (nbins <= 4096) return rfi_blocks_t<512, 8, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, s);
-    if (nbins <= 8192) return rfi_blocks_t<1024, 8, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, s);
-    if (nbins <= 16384) return rfi_blocks_t<1024, 16, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, s);
-    return rfi_blocks_t<1024, 0, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, s);
+                 size_t walk_smem, bool may_leave, cudaStream_t s) {
+    if (nbins <= 1024) return rfi_blocks_t<256, 4, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, may_leave, s);
+    if (nbins <= 4096) return rfi_blocks_t<512, 8, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, may_leave, s);
+    if (nbins <= 8192) return rfi_blocks_t<1024, 8, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, may_leave, s);
+    if (nbins <= 16384) return rfi_blocks_t<1024, 16, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, may_leave, s);
+    return rfi_blocks_t<1024, 0, PLAIN>(jobs, one, njobs, bs, nt, walk_smem, may_leave, s);
 }
 int rfi_blocks(int nbins, bool plain, const RfiJob* jobs, const RfiJob& one, int njobs, const pv::BeamStep* bs, int nt,
-               size_t walk_smem, cudaStream_t s) {
-    return plain ? rfi_blocks_p<true>(nbins, jobs, one, njobs, bs, nt, walk_smem, s)
-                 : rfi_blocks_p<false>(nbins, jobs, one, njobs, bs, nt, walk_smem, s);
+               size_t walk_smem, bool may_leave, cudaStream_t s) {
+    return plain ? rfi_blocks_p<true>(nbins, jobs, one, njobs, bs, nt, walk_smem, may_leave, s)
+                 : rfi_blocks_p<false>(nbins, jobs, one, njobs, bs, nt, walk_smem, may_leave, s);
 }
 
 }  // namespace
@@ -1067,6 +1092,8 @@ struct pv_rfi {
     int split = 1;  // rfi_shape's split of a wide beam over a cluster (the walk over spectra)
     bool walk = false;  // pv_rfi_set_split was called: the walk, spread as asked
     RfiWork work{};
+    long long started = 0;  // spectra run since the state was last set up, reset or loaded
+    int* h_hard = nullptr;  // RfiWork::hard
     float start_freq = 0.0f, end_freq = 0.0f;
     int nbins = 0;
     RfiConfig cfg{};
@@ -1088,6 +1115,8 @@ void free_device(pv_rfi* h) {
     if (h->d_terms) cudaFree(h->d_terms);
     if (h->d_killed) cudaFree(h->d_killed);
     if (h->work.rec) cudaFree(h->work.rec);  // one allocation
+    if (h->h_hard) cudaFreeHost(h->h_hard);
+    h->h_hard = nullptr;
     h->work = RfiWork{};
     h->dev = RfiBuffers{};
     h->d_terms = nullptr;
@@ -1170,7 +1199,17 @@ int setup(pv_rfi* h, int nbins, cudaStream_t s) {
         h->work.out = reinterpret_cast<SpecOut*>(p + sizeof(SpecRec) * kRfiBlock);
         h->work.hdr = reinterpret_cast<int*>(p + head);
         h->work.fill_at = h->work.hdr + kHdrWords;
+        PV_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h->h_hard), sizeof(int), cudaHostAllocMapped),
+                "allocate RFI block word");
+        *h->h_hard = 0;
+        h->work.hard = h->h_hard;
+        const size_t smem = rfi_walk_smem(nbins);
+        if (smem <= 227 * 1024)
+            PV_TRY(rfi_launch(pv_rfi_parts(nbins), 1, smem, 0, nullptr, nullptr, h->cfg, h->dev, nullptr, 0, 0, Geo{},
+                              nullptr, s));
     }
+    if (h->work.hdr) PV_CUDA(cudaMemsetAsync(h->work.hdr, 0, sizeof(int) * kHdrWords, s), "clear RFI block header");
+    h->started = 0;
     PV_CUDA(cudaMemcpyAsync(h->dev.state, &st, sizeof(st), cudaMemcpyHostToDevice, s), "copy RFI state");
     PV_CUDA(cudaMemsetAsync(h->dev.last_good, 0, sizeof(float) * nbins, s), "clear last good spectrum");
     PV_CUDA(cudaMemsetAsync(h->dev.mean_buf, 0, sizeof(double) * h->history, s), "clear history");
@@ -1259,8 +1298,13 @@ extern "C" int pv_rfi_run(pv_rfi* h, float* d_data, int nt, int nsub, int npol, 
     const Geo geo = make_geo(nsub, npol, nchan);
     if (rfi_in_blocks(h) && h->work.rec) {
         const RfiJob one{h->cfg, h->dev, d_data, d_flags, geo, h->work, nt, 0};
+        // while the histories may be filling under a bandpass with terms, or after a block with many spectra
+        // done over (as far as the GPU has got: the outputs do not depend on it)
+        const bool may_leave = (!rfi_flat(h->cfg, h->dev) && h->started < h->history) ||
+                               (h->h_hard && *static_cast<volatile int*>(h->h_hard) != 0);
+        h->started += nt;
         return rfi_blocks(nbins, rfi_plain(h->cfg, h->dev, npol), nullptr, one, 1, nullptr, nt, rfi_walk_smem(nbins),
-                          s);
+                          may_leave, s);
     }
     return rfi_launch(parts, h->split, smem, 1, nullptr, nullptr, h->cfg, h->dev, d_data, 0, nt, geo, d_flags, s);
 }
@@ -1274,6 +1318,7 @@ int pv::rfi_reset(pv_rfi* h, cudaStream_t s) {
     st.params0 = h->bp.params[0];
     st.bp_mean = Bandpass::at(h->bp.mean, h->bp.current.key());
     st.bp_rms = Bandpass::at(h->bp.rms, h->bp.current.key());
+    h->started = 0;
     // st is a stack value: copy synchronously with respect to the host
     PV_CUDA(cudaStreamSynchronize(s), "synchronise");
     PV_CUDA(cudaMemcpy(h->dev.state, &st, sizeof(st), cudaMemcpyHostToDevice), "reset RFI state");
@@ -1293,6 +1338,7 @@ long long pv::rfi_state_bytes(const pv_rfi* h, int nbins) {
 // no spectrum yet is set up first, so its initial state is what is saved.
 int pv::rfi_state_io(pv_rfi* h, int nbins, void* h_buf, bool save, cudaStream_t s) {
     PV_TRY(setup(h, nbins, s));
+    if (!save) h->started = 0;
     char* p = static_cast<char*>(h_buf);
     const size_t hist = sizeof(double) * (size_t)h->history;
     struct Part { void* dev; size_t bytes; };
@@ -1520,7 +1566,8 @@ int rfi_batch_ctas(const RfiBatch* b, int k) { return b->classes[k].njobs * b->c
 int rfi_batch_launch_one(RfiBatch* b, int k, cudaStream_t s) {
     auto& c = b->classes[k];
     if (c.njobs == 0) return PV_OK;
-    if (c.blocks) return rfi_blocks(c.nbins, c.plain, c.d_jobs, RfiJob{}, c.njobs, b->bs, b->nt, c.smem, s);
+    if (c.blocks) return rfi_blocks(c.nbins, c.plain, c.d_jobs, RfiJob{}, c.njobs, b->bs, b->nt, c.smem,
+                                    c.nbins > 4096 || !c.plain, s);
     return rfi_launch(c.parts, b->split, c.smem, c.njobs, c.d_jobs, b->bs, RfiConfig{}, RfiBuffers{}, nullptr, 0,
                       b->nt, Geo{}, nullptr, s);
 }

@@ -1,4 +1,4 @@
-// The clipper in blocks of spectra: three launches instead of a walk.
+// The clipper in blocks of spectra: a few launches instead of a walk.
 //
 // Included by rfi.cu inside its anonymous namespace, after RfiState,
 // RfiConfig, RfiBuffers, Geo and the reductions.
@@ -23,6 +23,7 @@
 //                    CTA with the exact state.
 //  rfi_apply_kernel  one CTA per spectrum: clips with the exact margin,
 //                    flattens, normalises and stores.
+//  rfi_kernel        the walk, for what the scan left to it.
 //
 // The margin moves over a block, and a channel whose value lies between the
 // expected and the exact margin fails the proof: rare in quiet data, common
@@ -41,6 +42,12 @@
 // (where the even neighbour depends on X).  So the rounded chain is a sum of
 // integers, and a prefix sum gives all of them at once.  A half-way case, or
 // a binade's end, is one of the spectra that are done over.
+//
+// A spectrum done over costs as much as a step of the walk or up to four times
+// that.  Where most of a block's spectra need it (the histories filling under a
+// bandpass with terms, spectra rejected one after another, averages that stay
+// 0, histories of a few spectra) the scan may leave the rest of the block to
+// the walk, which goes on from the state where the scan stopped (scan_leaves).
 //
 // Bound: reading the block (stats), again from L2 (apply) and writing it; the
 // scan is bound by the FP64 unit (each FP64 instruction of a warp takes its
@@ -71,6 +78,7 @@ struct RfiWork {
     SpecOut* out;  // [kRfiBlock]
     int* fill_at;  // [nbins] spectrum of the block that filled the channel's last good value (-1: earlier)
     int* hdr;      // see kHdr*
+    int* hard;     // kHdrHard of the last block for the host, in its memory
 };
 
 // Spectra per block: the block of a 3904-channel beam (32 MB) stays in L2
@@ -80,8 +88,11 @@ constexpr int kScanThreads = 512;
 constexpr int kZeroList = 2048;
 // RfiWork::hdr: before the block, num and the channels without a last good
 // value; after the first scan, the spectrum it reached, whether the second
-// pass is wanted and whether a spectrum of the block has filled channels.
-constexpr int kHdrNum = 0, kHdrZeros = 1, kHdrPos = 2, kHdrRedo = 3, kHdrFilled = 4, kHdrWords = 8;
+// pass is wanted and whether a spectrum of the block has filled channels; after
+// the last scan, the spectra that are done (the rest is the walk's) and whether
+// it left any or had many to do over one by one.
+constexpr int kHdrNum = 0, kHdrZeros = 1, kHdrPos = 2, kHdrRedo = 3, kHdrFilled = 4, kHdrEnd = 5, kHdrHard = 6,
+              kHdrWords = 8;
 // Failed proofs that the first scan does over by itself.  Each costs a scan of
 // one spectrum and a group begun again, a second pass 3 to 15 us of statistics:
 // the forecast at the first failure tells (more failures than kForecastMax,
@@ -454,7 +465,7 @@ struct ScanShared {
     float rf[kScanThreads], mf[kScanThreads], pi[kScanThreads], pb[kScanThreads];
     int first_bad;
     float dm, margin;
-    int sclip, fill, filled;
+    int fill, filled, rejected;
     float red[8 * 64], redm[8 * 32], redb[8 * 32];
     double fa[kSerial], fb[kSerial], fx[kSerial], ga[kSerial], gx[kSerial];
     int cnt[8];
@@ -613,6 +624,7 @@ __device__ __forceinline__ void scan_one(ScanShared& sh, const RfiConfig& cfg, c
             w.rec[i].total_good = total;
             w.out[i] = SpecOut{dm, margin, p0, (float)st.mean_run, sclip, {0, 0, 0}};
             sh.fill = fill;
+            sh.rejected = st.mean_size >= 1000 && sclip != 0 ? 1 : 0;
         }
     }
     __syncthreads();
@@ -1031,9 +1043,54 @@ __device__ __forceinline__ int scan_forecast(ScanShared& sh, const RfiConfig& cf
     return sh.first_bad;
 }
 
+// Spectra done over one by one in a scan so far, by why.
+struct ScanAlone {
+    int rejected, idle, other;  // idle: averages that are 0 (or not finite, or tiny)
+    __device__ __forceinline__ int all() const { return rejected + idle + other; }
+};
+
+// Whether the walk would do spectra i..n-1 sooner: more of them are expected to
+// be done over one by one than the walk's time is worth, as a part of them all.
+// While the histories fill under a bandpass with terms every one is.  Rejected
+// ones are counted in the records; others are taken to come on as often as
+// since spectrum i0, which takes many to believe unless the block before was
+// such a one.  us a spectrum by 64 / 512 / 1024 / 4096 / 8192 / 15616 channels:
+// walked 2.4 2.9 4.1 6.2 6.7 8.7, all rejected 2.8 3.1 3.8 5.2 8.5 19, every
+// fourth 9.2 9.2 9.8 11 14 20 for each rejected; with terms, walked 2.5 3.3 4.2
+// 6.2 6.8 9.0 and averages of 0 3.2 3.6 4.8 8.8 16 38; the histories filling
+// with terms, walked 5.9 6.8 8.7 14 15 19 and one by one 10 9.3 11 15 27 43.
+__device__ __forceinline__ bool scan_leaves(const ScanShared& sh, const RfiConfig& cfg, const RfiWork& w, bool flat,
+                                            int i0, int i, int n, const ScanAlone& alone) {
+    const RfiState& st = sh.st;
+    const int left = n - i, nbins = cfg.nbins;
+    if (left <= 16) return false;
+    if (!flat && st.rms_size < cfg.history) {
+        const float part = nbins > 512 && nbins <= 4096 ? 0.85f : 0.6f;
+        return (float)min(left, cfg.history - st.rms_size) >= part * (float)left;
+    }
+    const int done = alone.all();
+    if (done < 8 || (done & (done - 1)) != 0) return false;  // looked into at 8, 16, 32, ...
+    // parts of the spectra left from which on the walk is sooner (above 1: never)
+    const float part_rejected = nbins <= 512 ? 0.3f : (nbins <= 4096 ? 2.0f : 0.45f);
+    const float part_idle = nbins > 512 && nbins <= 4096 && !flat ? 0.8f : part_rejected;
+    int rejected = 0;
+    if (st.mean_size >= 1000) {
+        const float loud = narrow(st.mean_run) + cfg.sr * st.bp_rms * narrow(cfg.inv_sqrt_nbins);
+        for (int k = i; k < n; k += kScanThreads) {
+            const int j = k + (int)threadIdx.x;
+            rejected += __syncthreads_count(j < n && (w.rec[j].ssum > loud || w.rec[j].bad_bands >= 4));
+        }
+    }
+    const bool many = alone.idle + alone.other >= (w.hdr[kHdrHard] != 0 ? 32 : 512);
+    const float of_left = many ? (float)left / (float)(i - i0) : 0.0f;
+    return ((float)rejected + of_left * (float)alone.other) / part_rejected + of_left * (float)alone.idle / part_idle >=
+           (float)left;
+}
+
 template <int P>
 __device__ __forceinline__ void rfi_scan_body(const RfiConfig& cfg, const RfiBuffers& bufs, const RfiWork& w,
-                                              const float* __restrict__ rows, const Geo& geo, int n, bool second) {
+                                              const float* __restrict__ rows, const Geo& geo, int n, bool second,
+                                              bool may_leave) {
     __shared__ ScanShared sh;
     const int tid = threadIdx.x;
     const long long spec_elems = (long long)geo.nsub * geo.npol * geo.nchan;
@@ -1057,6 +1114,8 @@ __device__ __forceinline__ void rfi_scan_body(const RfiConfig& cfg, const RfiBuf
         else if (filled)
             list_zeros(sh, cfg, bufs);
     }
+    const int i0 = i;
+    ScanAlone by_itself{0, 0, 0};
     int alone = 0, streak = 0;     // spectra to do one by one before the next group
     int serial = 0, grow = 32;     // spectra of the next group if its averages are added one by one
     int failed = 0;
@@ -1075,7 +1134,9 @@ __device__ __forceinline__ void rfi_scan_body(const RfiConfig& cfg, const RfiBuf
             else m = min(m, H);
             // averages that are 0, not finite or tiny have no usable binade
             const RfiState& st = sh.st;
-            if (!binade64(rs < H ? st.rms_acc : st.rms_run).ok || !binade64(rs < H ? st.mean_acc : st.mean_run).ok) m = 0;
+            const bool idle =
+                !binade64(rs < H ? st.rms_acc : st.rms_run).ok || !binade64(rs < H ? st.mean_acc : st.mean_run).ok;
+            if (idle) m = 0;
             if (alone > 0) {
                 --alone;
                 m = 0;
@@ -1107,8 +1168,12 @@ __device__ __forceinline__ void rfi_scan_body(const RfiConfig& cfg, const RfiBuf
                 streak = f == 0 ? min(streak + 1, 6) : 0;
                 alone = f == 0 ? (1 << streak) - 1 : 0;
             }
+            if (may_leave && scan_leaves(sh, cfg, w, flat, i0, i, n, by_itself)) break;
             scan_one<P>(sh, cfg, bufs, w, rows + (long long)i * spec_elems, geo, i);
             filled |= sh.fill != 0 && sh.filled != 0;
+            if (sh.rejected) ++by_itself.rejected;
+            else if (idle) ++by_itself.idle;
+            else ++by_itself.other;
             ++i;
         }
         if (!ask) break;
@@ -1135,7 +1200,16 @@ __device__ __forceinline__ void rfi_scan_body(const RfiConfig& cfg, const RfiBuf
     }
     __syncthreads();
     if (tid == 0) {
-        if (!redo) *bufs.state = sh.st;
+        if (!redo) {
+            *bufs.state = sh.st;
+            w.hdr[kHdrEnd] = i;
+            const int done = by_itself.all();
+            const int hard = i < n || (done >= 32 && 10 * done >= 3 * (i - i0)) ? 1 : 0;
+            if (w.hdr[kHdrHard] != hard) {
+                w.hdr[kHdrHard] = hard;
+                if (w.hard) *w.hard = hard;
+            }
+        }
         if (!second) {
             w.hdr[kHdrPos] = i;
             w.hdr[kHdrRedo] = redo ? 1 : 0;
@@ -1151,7 +1225,10 @@ __device__ __forceinline__ void rfi_scan_body(const RfiConfig& cfg, const RfiBuf
 template <int P, int KM, bool PLAIN>
 __device__ __forceinline__ void rfi_apply_body(const RfiConfig& cfg, const RfiBuffers& bufs, const RfiWork& w,
                                                float* __restrict__ row, const Geo& geo,
-                                               unsigned char* __restrict__ flags, int i, bool last) {
+                                               unsigned char* __restrict__ flags, int i) {
+    const int end = w.hdr[kHdrEnd];
+    if (i >= end) return;
+    const bool last = i == end - 1;
     constexpr int NW = P / 32;
     __shared__ float red[32 * 2];
     __shared__ float s_norm[2];
@@ -1247,7 +1324,8 @@ __device__ __forceinline__ void rfi_apply_body(const RfiConfig& cfg, const RfiBu
 // The running fraction of bad channels (RFI_Clipper.cpp:345-352,548-560), one
 // FP32 add per spectrum in order, by one CTA beside those of the spectra.
 template <int P>
-__device__ __forceinline__ void rfi_fraction(const RfiConfig& cfg, const RfiBuffers& bufs, const RfiWork& w, int n) {
+__device__ __forceinline__ void rfi_fraction(const RfiConfig& cfg, const RfiBuffers& bufs, const RfiWork& w) {
+    const int n = w.hdr[kHdrEnd];
     __shared__ __align__(16) float f[P];
     const int period = 10 * cfg.history, tid = threadIdx.x;
     // the statistics' reset is after the spectrum at which num is 0

@@ -166,3 +166,45 @@ def test_few_spectra_take_one_launch(pv, oracle, cuda, nsub, few):
         before = pv.launches()
         g.run(d[:n])
         assert pv.launches() - before == want
+
+
+@pytest.mark.parametrize("nsub,nchan,kind", [
+    (8, 16, "rejected"), (8, 16, "zeros"), (8, 16, "terms"), (320, 16, "rejected"), (513, 16, "rejected"),
+    (513, 16, "zeros"), (513, 16, "terms"), (128, 16, "terms"), (1025, 16, "rejected"), (8, 16, "burst"),
+])
+def test_blocks_left_to_the_walk(pv, oracle, cuda, nsub, nchan, kind):
+    """Spectra that a scan does over one by one, most of a block's: it leaves
+    the rest to the walk, from the block's start, its middle, and not at all
+    where the rest is quiet; the blocks after it go on from there."""
+    rng = np.random.default_rng(nsub + len(kind))
+    nbins, H = nsub * nchan, 1100
+    nt = H + 3000
+    data = stokes_filterbank(rng, nt, nsub, nchan)
+    bp = make_bp_text(nbins, START, WIDTH, 1000.0, 50.0, (0.3,) if kind == "terms" else ())
+    if kind == "rejected":  # two calls are left to the walk; quiet; then every third
+        data[H + 300:H + 1450] *= 2.0
+        data[H + 1900::3] *= 2.0
+    elif kind == "burst":  # 70 spectra, then quiet
+        data[H + 300:H + 370] *= 2.0
+    elif kind == "zeros":
+        data[:H + 900] = 0.0
+    _run(pv, oracle, cuda, data, (700, H + 100, H + 600, H + 1100, H + 1600, H + 2600), bp, H)
+
+
+def test_polarisations_of_blocks_left_to_the_walk(pv, oracle, cuda):
+    import torch
+    rng = np.random.default_rng(2)
+    nt, nsub, npol, nchan = 2500, 8, 4, 16
+    data = rng.normal(1000.0, 50.0, (nt, nsub, npol, nchan)).astype(np.float32)
+    data[:, 3, 0, 5] *= 20.0
+    data[1200:] *= 2.0
+    bp = make_bp_text(nsub * nchan, START, WIDTH, 1000.0, 50.0)
+    kw = dict(cr=5.0, sr=4.0, history=1100, zero_dming=True)
+    outs = []
+    for split in (None, 0):  # in blocks, and walked throughout
+        d = torch.from_numpy(data).to(cuda)
+        r = pv.RFI(bp, split=split, **kw)
+        f = [r.run(d[a:b], flags=True).cpu().numpy() for a, b in ((0, 1500), (1500, 2000), (2000, nt))]
+        outs.append((d.cpu().numpy(), np.concatenate(f)))
+    assert np.array_equal(outs[0][0], outs[1][0]) and np.array_equal(outs[0][1], outs[1][1])
+    assert (outs[0][1][1300:] & 2).all()

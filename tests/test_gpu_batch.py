@@ -286,3 +286,52 @@ def test_batch_of_twelve_beams_in_three_clipper_classes_equals_beams_alone(pv, c
     parts = {pv.load().pv_rfi_parts(ns * nc) for ns, nc in shapes}
     assert len(parts) == 3
     _compare_with_beams_alone(pv, cuda, mix, False, True, 0, True, True)
+
+
+@pytest.mark.parametrize("graph,pipelined", [(True, False), (True, True), (False, True)])
+def test_batch_of_blocks_and_walked_clippers(pv, cuda, mix_configs, graph, pipelined):
+    """Beams whose clippers are done in blocks beside beams whose RMS does not
+    come from the mean and whose spectra are walked, two channel counts of
+    each, and one whose bandpass has terms: in a pipelined batch the blocks
+    come first and the walk runs beside the dedispersion."""
+    rng = np.random.default_rng(97)
+    walked = calibrated(pv, cuda, beam_kw(5, 16, 24, 0.6, rms_from_mean=0), rng)      # 80 channels
+    walked2 = calibrated(pv, cuda, beam_kw(40, 32, 24, 0.05, rms_from_mean=0), rng)   # 1280 channels
+    blocks2 = calibrated(pv, cuda, beam_kw(40, 32, 16, 0.05), rng)
+    kw = beam_kw(6, 32, 24, 0.3)
+    lo, nbins = kw["fch1"], 6 * 32
+    terms = pv.beam_config(**dict(kw, bp_text=make_bp_text(nbins, lo, abs(kw["foff"]), 500.0, 300.0, (0.05,))))
+    _compare_with_beams_alone(pv, cuda, [mix_configs[0], walked, blocks2, walked2, terms], False, graph, 0, False,
+                              pipelined)
+
+
+def test_batch_wide_clipper_alone_on_a_cluster(pv, cuda, mix_configs):
+    """An unpipelined batch with its walked 5120-channel beam on 4 CTAs."""
+    rng = np.random.default_rng(96)
+    wide = calibrated(pv, cuda, beam_kw(80, 64, 16, 0.02), rng)
+    _compare_with_beams_alone(pv, cuda, mix_configs[:1] + [wide], False, True, 0, False, False, rfi_cluster4=True)
+
+
+def test_batch_of_rejected_spectra_equals_beams_alone(pv, cuda):
+    """A wide beam and a narrow one whose every spectrum after the first chunks
+    is rejected: the batch's blocks leave theirs to the walk."""
+    import torch
+    rng = np.random.default_rng(95)
+    cfgs = [calibrated(pv, cuda, beam_kw(n, 64, d, s, sr=0.5), rng) for n, d, s in ((80, 16, 0.02), (4, 64, 1.0))]
+    batch = pv.Batch(cfgs, tune=False, graph=True)
+    alone = [pv.Beam(c) for c in cfgs]
+    for step in range(6):
+        for i, c in enumerate(cfgs):
+            v16, _ = voltages(rng, c.nsub, 2, c.chunk * 4 * c.nchan_sub)
+            v16 = (v16 * (1 if step < 3 else 2)).astype(np.int16)
+            x = torch.from_numpy(v16.reshape(c.nsub, 2, -1)).to(cuda)
+            batch.set_input(i, x)
+            alone[i].process(x)
+        batch.run()
+        torch.cuda.synchronize()
+        for i, c in enumerate(cfgs):
+            shape = (c.chunk, c.nsub * c.nchan_sub)
+            a = pv.device_array(alone[i].buffers()[0], shape).cpu().numpy()
+            assert np.array_equal(pv.device_array(batch.buffers(i)[0], shape).cpu().numpy(), a)
+            if step > 3:  # rejected: -0.2 less the bandpass, the same for every channel
+                assert (a == a[:, :1]).mean() > 0.9

@@ -208,3 +208,25 @@ def test_polarisations_of_blocks_left_to_the_walk(pv, oracle, cuda):
         outs.append((d.cpu().numpy(), np.concatenate(f)))
     assert np.array_equal(outs[0][0], outs[1][0]) and np.array_equal(outs[0][1], outs[1][1])
     assert (outs[0][1][1300:] & 2).all()
+
+
+@pytest.mark.parametrize("nsub", [8, 128])
+@pytest.mark.parametrize("terms", [(), (0.3,)])
+def test_rms_of_each_spectrum(pv, oracle, cuda, nsub, terms):
+    """Without computeRMSfromMean the RMS is each spectrum's own after
+    flattening, and the spectra are walked, one launch a call."""
+    import torch
+    nt, nchan = 2600, 16
+    data = stokes_filterbank(np.random.default_rng(nsub), nt, nsub, nchan)
+    bp = make_bp_text(nsub * nchan, START, WIDTH, 1000.0, 50.0, terms)
+    kw = dict(cr=5.0, sr=4.0, history=1100, zero_dming=True, mean_over_rms=False)
+    g = pv.RFI(bp, **kw)
+    o = oracle.RFI(bp, mode=1, parts=pv.load().pv_rfi_parts(nsub * nchan), **kw)
+    for a, b in ((0, 1), (1, 1500), (1500, nt)):
+        d = np.ascontiguousarray(data[a:b])
+        dd = torch.from_numpy(d).to(cuda)
+        before = pv.launches()
+        gf = g.run(dd, flags=True).cpu().numpy()
+        assert pv.launches() - before == 1
+        assert np.array_equal(gf, o.run(d, flags=True))
+        assert np.array_equal(dd.cpu().numpy(), d)

@@ -890,15 +890,28 @@ __global__ void __launch_bounds__(P, P == 256 ? 6 : (P == 512 ? 3 : 1)) rfi_appl
 }
 
 // The clippers of many beams at once: cluster b (CTAs b*C .. b*C+C-1) runs
-// spectra [t0, t0 + n) of job b (every job of a launch has the same partial
-// count), or with rest what the scan of that block left; beams without a chunk
-// this step return at once.
+// job b (every job of a launch has the same partial count); beams without a
+// chunk this step return at once.
 template <int T, int C>
 __global__ void __launch_bounds__(T, 1) rfi_batch_kernel(const RfiJob* __restrict__ jobs,
-                                                         const pv::BeamStep* __restrict__ bs, int t0, int n,
-                                                         bool rest) {
+                                                         const pv::BeamStep* __restrict__ bs) {
     const int job = blockIdx.x / C;
     if (bs && !bs[jobs[job].beam].active) return;  // the whole cluster returns
+    const RfiConfig cfg = jobs[job].cfg;
+    const RfiBuffers bufs = jobs[job].bufs;
+    const Geo geo = jobs[job].geo;
+    rfi_body<T, C>(cfg, bufs, jobs[job].data, jobs[job].nt, geo, jobs[job].flags, (int)(blockIdx.x % C));
+}
+
+// The same of beams done in blocks: spectra [t0, t0 + n), or with rest what the
+// scan of that block left.  (A kernel of its own: the range costs the 1024
+// threads of rfi_batch_kernel<1024, 1> registers, 7 % of their time.)
+template <int T, int C>
+__global__ void __launch_bounds__(T, 1) rfi_batch_part_kernel(const RfiJob* __restrict__ jobs,
+                                                              const pv::BeamStep* __restrict__ bs, int t0, int n,
+                                                              bool rest) {
+    const int job = blockIdx.x / C;
+    if (bs && !bs[jobs[job].beam].active) return;
     const RfiConfig cfg = jobs[job].cfg;
     const RfiBuffers bufs = jobs[job].bufs;
     const Geo geo = jobs[job].geo;
@@ -966,21 +979,29 @@ int rfi_launch_ex(K kern, int clusters, int C, int T, size_t smem, cudaStream_t 
     return PV_OK;
 }
 
-// Sets the shared-memory attribute of both kernels of a shape and launches
-// one of them on spectra [t0, t0 + nt): jobs != null selects the batched
-// kernel (nblocks jobs; nblocks == 0: the attributes only, before any stream
-// capture).  rest: only what the scan of these spectra left (hdr: of the one
-// beam).
+// Sets the shared-memory attribute of the kernels of a shape and launches one
+// of them: jobs != null selects the batched kernel (nblocks jobs; nblocks ==
+// 0: the attributes only, before any stream capture).  part: spectra [t0, t0 +
+// nt) of jobs done in blocks; a batch's other jobs run whole.  rest: only what
+// the scan of these spectra left (hdr: of the one beam).
 template <int T, int C>
 int rfi_launch_t(size_t smem, int nblocks, const RfiJob* jobs, const pv::BeamStep* bs,
                  const RfiConfig& cfg, const RfiBuffers& bufs, float* data, int t0, int nt, const Geo& geo,
-                 unsigned char* flags, cudaStream_t s, bool rest, const int* hdr) {
+                 unsigned char* flags, cudaStream_t s, bool part, bool rest, const int* hdr) {
+    constexpr bool kParts = C == 4 ? T == 256 : T <= 512;  // rfi_shape's split 1, which blocks take
     if (nblocks == 0) {
+        if constexpr (kParts) PV_TRY(rfi_set_smem(rfi_batch_part_kernel<T, C>, smem));
         PV_TRY(rfi_set_smem(rfi_kernel<T, C>, smem));
         return rfi_set_smem(rfi_batch_kernel<T, C>, smem);
     }
+    if constexpr (kParts) {
+        if (jobs && part) {
+            PV_TRY(rfi_launch_ex(rfi_batch_part_kernel<T, C>, nblocks, C, T, smem, s, jobs, bs, t0, nt, rest));
+            return pv::check_launch("rfi_batch_part_kernel");
+        }
+    }
     if (jobs) {
-        PV_TRY(rfi_launch_ex(rfi_batch_kernel<T, C>, nblocks, C, T, smem, s, jobs, bs, t0, nt, rest));
+        PV_TRY(rfi_launch_ex(rfi_batch_kernel<T, C>, nblocks, C, T, smem, s, jobs, bs));
         return pv::check_launch("rfi_batch_kernel");
     }
     if (!rest) PV_TRY(rfi_set_smem(rfi_kernel<T, C>, smem));  // of a rest: set by setup()
@@ -993,12 +1014,13 @@ int rfi_launch_t(size_t smem, int nblocks, const RfiJob* jobs, const pv::BeamSte
 
 int rfi_launch(int parts, int split, size_t smem, int nblocks, const RfiJob* jobs, const pv::BeamStep* bs,
                const RfiConfig& cfg, const RfiBuffers& bufs, float* data, int t0, int nt, const Geo& geo,
-               unsigned char* flags, cudaStream_t s, bool rest = false, const int* hdr = nullptr) {
+               unsigned char* flags, cudaStream_t s, bool part = false, bool rest = false,
+               const int* hdr = nullptr) {
     int T = 0, C = 0;
     rfi_shape(parts, split, &T, &C);
 #define PV_RFI_SHAPE(TT, CC)                                                                          \
     if (T == TT && C == CC)                                                                          \
-        return rfi_launch_t<TT, CC>(smem, nblocks, jobs, bs, cfg, bufs, data, t0, nt, geo, flags, s, rest, hdr);
+        return rfi_launch_t<TT, CC>(smem, nblocks, jobs, bs, cfg, bufs, data, t0, nt, geo, flags, s, part, rest, hdr);
     PV_RFI_SHAPE(256, 1)
     PV_RFI_SHAPE(512, 1)
     PV_RFI_SHAPE(1024, 1)
@@ -1030,7 +1052,7 @@ int rfi_blocks_t(const RfiJob* jobs, const RfiJob& one, int njobs, const pv::Bea
         const int n = std::min(kRfiBlock, nt - t0);
         if (n <= rfi_walk_few(P)) {
             PV_TRY(rfi_launch(P, 1, walk_smem, njobs, jobs, bs, one.cfg, one.bufs, one.data, t0, n, one.geo, one.flags,
-                              s));
+                              s, true));
             continue;
         }
         for (int second = 0; second < 2; ++second) {
@@ -1044,7 +1066,7 @@ int rfi_blocks_t(const RfiJob* jobs, const RfiJob& one, int njobs, const pv::Bea
         PV_TRY(pv::check_launch("rfi_apply_kernel"));
         if (may_leave)
             PV_TRY(rfi_launch(P, 1, walk_smem, njobs, jobs, bs, one.cfg, one.bufs, one.data, t0, n, one.geo, one.flags,
-                              s, true, one.work.hdr));
+                              s, true, true, one.work.hdr));
     }
     return PV_OK;
 }

@@ -1065,7 +1065,12 @@ __device__ __forceinline__ bool scan_leaves(const ScanShared& sh, const RfiConfi
     const int left = n - i, nbins = cfg.nbins;
     if (left <= 16) return false;
     if (!flat && st.rms_size < cfg.history) {
-        const float part = nbins > 512 && nbins <= 4096 ? 0.85f : 0.6f;
+        const float part = nbins <= 128    ? 0.37f
+                           : nbins <= 512  ? 0.45f
+                           : nbins <= 1024 ? 0.65f
+                           : nbins <= 4096 ? 0.85f
+                           : nbins <= 8192 ? 0.45f
+                                           : 0.35f;
         return (float)min(left, cfg.history - st.rms_size) >= part * (float)left;
     }
     const int done = alone.all();

@@ -326,13 +326,14 @@ int pv_rfi_bandpass_current(pv_rfi* rfi, float* h_out, int nbins, float* h_stats
  * band of nbins channels (256, 512 or 1024): partial p sums channels p,
  * p + parts, ... in order. */
 int pv_rfi_parts(int nbins);
-/* Makes pv_rfi_run walk the spectra one after another, and how that spreads a
- * band over the GPU (no counterpart in the reference, whose clipper is one
- * CPU thread): 0 one CTA of `parts` threads; 1 bands of 1024 partials over a
+/* Makes pv_rfi_run walk the spectra one after another for the rest of the
+ * clipper's life, and how that spreads a band over the GPU (no counterpart in
+ * the reference, whose clipper is one CPU thread): 0 one CTA of `parts` threads; 1 bands of 1024 partials over a
  * cluster of 4 CTAs of 256 threads; 2 bands of 512 or 1024 partials over
  * clusters of 128-thread CTAs.  Without this call a clipper whose RMS comes
- * from the mean (compute_rms_from_mean) does its spectra in blocks, and one
- * whose RMS does not walks them as with 1.  Every choice computes the same
+ * from the mean (compute_rms_from_mean) does its spectra in blocks (a few
+ * spectra, and those that a block would do one by one anyway, it walks as
+ * with 1), and one whose RMS does not walks them as with 1.  Every choice computes the same
  * partial sums, so flags and outputs are identical. */
 int pv_rfi_set_split(pv_rfi* rfi, int split);
 

@@ -3,13 +3,13 @@
 // each stage of all beams in as few launches as the kernels allow:
 //
 //   K1  chan_stokes_seg_kernel one launch per channels-per-subband class
-//   K2  the clipper in blocks  three to five launches per block of 2048 spectra
+//   K2  the clipper in blocks  five or six launches per block of 2048 spectra
 //                              and channel count (rfi_batch_kernel, one CTA or
 //                              cluster per beam, where the clipper is walked)
 //   A8  ring_write_batch_kernel one launch
 //   K4  dedisperse_batch_kernel one persistent launch over every beam's tiles,
 //                              DM x time tile shape chosen by the autotuner
-//   K5  analyser               per beam (count, scan, emit)
+//   K5  analyser               per beam (count, emit)
 //
 // Pipelined mode (PV_BATCH_PIPELINED): a step clips and ring-writes chunk k
 // and dedisperses and searches window k-lag-1, complete since the previous

@@ -47,7 +47,7 @@ bool chan_fast_supported(int nchan, int ntaps, int npol, int nstokes, int window
 // pkt_bytes > 0 (the register channeliser only)
 int channelise_stokes_i(pv_ppf* h, const void* d_in, int nsub, int nblocks, int window, int bin, float* d_stokes,
                         int* nu_out, long long pkt_bytes, int pkt_nsub, cudaStream_t s);
-// chan_stokes_seg_kernel takes the job (voltages, not packets; N channels)
+// chan_stokes_seg_kernel takes the job (voltages or packets; N channels)
 bool chan_seg_supported(int nchan, const ChanJob& job);
 // Sets range and nranges for `parts` such jobs side by side in one launch; returns the job's warps
 // (seg: CTAs).

@@ -5,10 +5,11 @@
 // channel-clip margin, bandpass level and rejection test depend on running
 // averages updated by the previous spectrum.  With the RMS taken from the mean
 // (computeRMSfromMean, the default) the spectra are done in blocks, all of a
-// block's spectra at once (rfi_blocks.cuh: 0.24 ms for 4096 spectra of 3904
-// channels).  Without it, or when a spread over CTAs is asked for, they are
-// walked (rfi_body: 24 ms): one CTA, or for a wide beam a cluster of CTAs,
-// takes a beam's spectra in order.  In both, partial p (P = 256, 512
+// block's spectra at once (rfi_blocks.cuh: 4096 spectra of 3904 channels in
+// 0.32 ms, 0.23 where no proof fails, as in a chunk run again).  Without it,
+// when a spread over CTAs is asked for, for calls of a few spectra and for what
+// a block leaves, they are walked (rfi_body: 24 ms): one CTA, or for a wide
+// beam a cluster of CTAs, takes a beam's spectra in order.  In both, partial p (P = 256, 512
 // or 1024 by channel count) owns channels p, p+P, ... of each spectrum.  The
 // state (running mean/RMS, their history rings, the last good spectrum, the
 // bandpass offset) lives in device memory between calls, so a stream of
